@@ -39,6 +39,7 @@
 #include <cuda.h>  // CUcontext / CUresult types; the two driver calls are looked up at run time
 
 #include "../../include/xenodon.h"
+#include "xn_bricks.h"
 #include "xn_ctx.h"
 #include "xn_internal.h"
 #include "xn_scan.cuh"
@@ -51,27 +52,6 @@ using namespace scan;
 constexpr uint32_t LEAF = 0x80000000u;
 constexpr uint64_t NONE = ~0ull;
 constexpr uint8_t F_LEAF = 1, F_INSIDE = 2, F_AMBIG = 4;
-
-struct LevelGeom {
-    uint32_t bx, by, bz;  // box of stored cells
-    uint64_t n;           // bx*by*bz
-    uint64_t e;           // cell extent in voxels
-};
-
-struct CDStats {  // ChannelDiff: sums, per-channel min and max (packed RGBA)
-    unsigned long long sum[4];
-    uint32_t mn, mx;
-};
-
-struct SDStats {  // StdDev: first and second moments
-    unsigned long long s1[4];
-    unsigned long long s2[4];
-};
-
-struct GridDev {
-    const uint32_t* vox;  // packed RGBA8, x fastest
-    uint32_t dx, dy, dz;
-};
 
 __device__ __forceinline__ uint32_t vox_at(const GridDev& g, uint32_t x, uint32_t y, uint32_t z) {
     return __ldg(g.vox + (uint64_t)x + (uint64_t)g.dx * ((uint64_t)y + (uint64_t)g.dy * z));
@@ -104,7 +84,6 @@ struct UpArgs {
     double stddev;          // StdDev threshold
     unsigned int* ambig_count;
     unsigned long long* ambig_list;
-    int lean;               // subtree sizes count internal nodes only (the lean build)
 };
 
 __device__ __forceinline__ void cell_coords(uint64_t i, const LevelGeom& L, uint32_t& x, uint32_t& y, uint32_t& z) {
@@ -120,7 +99,7 @@ __device__ __forceinline__ uint64_t cell_index(const LevelGeom& L, uint32_t x, u
 
 // Subtree size of child k of an internal cell (x, y, z) of the current level.
 __device__ __forceinline__ uint64_t child_size(const UpArgs& a, uint32_t x, uint32_t y, uint32_t z, int k) {
-    if (a.child_is_voxel) return a.lean ? 0 : 1;
+    if (a.child_is_voxel) return 1;
     uint32_t cx = 2 * x + ((k >> 2) & 1), cy = 2 * y + ((k >> 1) & 1), cz = 2 * z + (k & 1);
     return a.child_size[cell_index(a.child, cx, cy, cz)];
 }
@@ -136,7 +115,7 @@ __global__ void up_level_kernel(UpArgs a) {
     const uint64_t ox = x * e, oy = y * e, oz = z * e;
     const bool inside = ox < a.g.dx && oy < a.g.dy && oz < a.g.dz;
     if (!inside) {  // OctreeConstruction.h:146-154
-        a.size[i] = a.lean ? 0 : 1;
+        a.size[i] = 1;
         a.color[i] = 0;
         a.flags[i] = F_LEAF;
         return;
@@ -225,7 +204,7 @@ __global__ void up_level_kernel(UpArgs a) {
     }
     const bool leaf = (!split && fully) || e == 1;
     a.flags[i] = (leaf ? F_LEAF : 0) | F_INSIDE | (ambiguous ? F_AMBIG : 0);
-    uint64_t sz = leaf && a.lean ? 0 : 1;
+    uint64_t sz = 1;
     if (!leaf) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) sz += child_size(a, x, y, z, k);
@@ -273,7 +252,7 @@ __global__ void resize_level_kernel(UpArgs a) {
     uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= a.cur.n) return;
     if (a.flags[i] & F_LEAF) {
-        a.size[i] = a.lean ? 0 : 1;
+        a.size[i] = 1;
         return;
     }
     uint32_t x, y, z;
@@ -293,8 +272,6 @@ struct DownArgs {
     const unsigned long long* child_size;
     const uint32_t* color;
     const uint8_t* flags;
-    const uint32_t* child_color;  // lean build: the child level's colours and flags
-    const uint8_t* child_flags;
     const unsigned long long* start;
     unsigned long long* child_start;
     uint32_t* nodes;  // n_total x 10 words, or null when only the starts are wanted
@@ -375,68 +352,12 @@ __global__ void down_level_kernel(DownArgs a) {
     }
 }
 
-// The lean build's top-down pass: sizes and starts count internal nodes only,
-// so index N - start - size is a node's rank among the internal nodes in the
-// reference's node order -- the order the device layout (svo_layout.cu) gives
-// them.  Every internal cell writes its eight child words (leaf: bit 31 | RGB,
-// internal: that child's rank) and its depth; leaves write nothing.
-__global__ void lean_down_kernel(DownArgs a, uint32_t* inner, uint32_t* inner_depth) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    unsigned long long leaves = 0, internal = 0;
-    unsigned int deepest = 0;
-    const uint64_t st = i < a.cur.n ? a.start[i] : NONE;
-    if (st != NONE && !(a.flags[i] & F_LEAF)) {
-        internal = 1;
-        const uint64_t idx = a.n_total - st - a.size[i];
-        uint32_t x, y, z;
-        cell_coords(i, a.cur, x, y, z);
-        uint64_t run = st;
-        uint32_t ch[8];
-        for (int k = 0; k < 8; ++k) {
-            const uint32_t cx = 2 * x + ((k >> 2) & 1), cy = 2 * y + ((k >> 1) & 1), cz = 2 * z + (k & 1);
-            if (a.child_is_voxel) {
-                const uint32_t v = (cx < a.g.dx && cy < a.g.dy && cz < a.g.dz) ? vox_at(a.g, cx, cy, cz) : 0u;
-                ch[k] = LEAF | (v & 0xFFFFFFu);
-                ++leaves;
-            } else {
-                const uint64_t ci = cell_index(a.child, cx, cy, cz);
-                if (a.child_flags[ci] & F_LEAF) {
-                    ch[k] = LEAF | (a.child_color[ci] & 0xFFFFFFu);
-                    ++leaves;
-                } else {
-                    const uint64_t cS = a.child_size[ci];
-                    a.child_start[ci] = run;
-                    ch[k] = (uint32_t)(a.n_total - run - cS);
-                    run += cS;
-                }
-            }
-        }
-        deepest = leaves ? (unsigned)a.depth + 1 : 0;
-        uint4* p = reinterpret_cast<uint4*>(inner + idx * 8);
-        p[0] = make_uint4(ch[0], ch[1], ch[2], ch[3]);
-        p[1] = make_uint4(ch[4], ch[5], ch[6], ch[7]);
-        inner_depth[idx] = (uint32_t)a.depth;
-    }
-    for (int o = 16; o > 0; o >>= 1) {
-        leaves += __shfl_down_sync(0xFFFFFFFFu, leaves, o);
-        internal += __shfl_down_sync(0xFFFFFFFFu, internal, o);
-        deepest = max(deepest, __shfl_down_sync(0xFFFFFFFFu, deepest, o));
-    }
-    if ((threadIdx.x & 31) == 0) {
-        if (leaves) atomicAdd(a.leaves, leaves);
-        if (internal) atomicAdd(a.existing + 1, internal);
-        if (deepest) atomicMax(a.max_depth, deepest);
-    }
-}
-
 struct LevelDev {
     LevelGeom geom;
     const unsigned long long* size;
     const unsigned long long* start;
     const uint8_t* flags;
 };
-
-constexpr int MAX_LEVELS = 40;
 
 struct RopeArgs {
     int L;  // depth of single-voxel cells
@@ -741,12 +662,96 @@ int exclusive_scan(Scratch& sc, const In* in, uint64_t n, unsigned* out, cudaStr
 
 }  // namespace
 
+// The build over bricks (svo_bricks.cu), for sparse and rope trees of at least
+// 16 voxels on the longest side: the node array, or with `layout` the volume's
+// device arrays.
+int build_bricks(Ctx* c, const GridDev& g, uint64_t side, int L, bool ropes, int heuristic, double threshold,
+                 uint32_t** d_nodes, uint64_t* d_nodes_bytes, xn_build_stats* stats, Volume* layout, bool lean,
+                 SubBuild* sub) {
+    cudaStream_t s = c->stream;
+    Scratch sc(c);
+    BrickBuild b{};
+    b.g = g;
+    b.L = L;
+    b.heuristic = heuristic;
+    b.chan_diff = (uint32_t)(uint8_t)threshold;
+    b.stddev = threshold;
+    b.sequential = heuristic == XN_HEUR_STD_DEV && getenv("XN_BUILD_STDDEV_SEQUENTIAL") != nullptr;
+    const uint64_t bytes = brick_plan(b, side, nullptr);
+    if (b.geo[b.Lb].n > 0x7FFFFFFFull) return fail(XN_ERR_ARG, "xn_build_svo: grid too large");
+    unsigned char* base = nullptr;
+    int r;
+    if ((r = sc.alloc(&base, bytes, "xn_build_svo: scratch"))) return r;
+    brick_plan(b, side, base);
+    cudaError_t e = brick_scan(b, s);
+    const uint64_t stat_bytes = heuristic == XN_HEUR_STD_DEV ? sizeof(SDStats) : sizeof(CDStats);
+    if (e == cudaSuccess && sub) e = cudaMemcpyAsync(sub->root_stats, b.stats, stat_bytes, cudaMemcpyDeviceToHost, s);
+    unsigned long long info[2] = {0, 0};
+    if (e == cudaSuccess) e = cudaMemcpyAsync(info, b.info, sizeof info, cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) return cuda_fail(e, "xn_build_svo: bottom-up pass");
+    const uint64_t Ni = info[0], n_total = 8 * Ni + 1, n_leaves = 7 * Ni + 1;
+    if (layout && Ni == 0) return LEAN_LEAF_ROOT;
+    if (lean && Ni >= LEAF) return fail(XN_ERR_FORMAT, "xn_build_svo: more than 2^31 internal nodes");
+    if (!lean && n_total > 0xFFFFFFFFull)
+        return fail(XN_ERR_FORMAT, "xn_build_svo: %llu nodes exceed the 32-bit node indices of the SVO format",
+                    (unsigned long long)n_total);
+    if (layout && !lean && n_leaves >= ROPE_EXIT - LEAF)
+        return fail(XN_ERR_FORMAT, "octree layout: more than 2^31 internal nodes or leaves");
+    BrickOut out{};
+    if (layout) {
+        layout->n_inner = Ni;
+        layout->n_leaves = lean ? 0 : n_leaves;
+        auto take = [&](uint32_t** p, uint64_t n, const char* what) {
+            return c->device_alloc(reinterpret_cast<void**>(p), n, what);
+        };
+        r = take(&layout->inner, Ni * 32, "xn_build_svo: inner nodes");
+        if (!r) r = take(&layout->inner_depth, Ni * 4, "xn_build_svo: inner depths");
+        if (!r && !lean) r = take(&layout->rinner, Ni * 32, "xn_build_svo: rope inner nodes");
+        if (!r && !lean) r = take(&layout->leaves, n_leaves * 32, "xn_build_svo: leaves");
+        if (r) {
+            layout->release_layout();
+            return r;
+        }
+        out.inner = layout->inner;
+        out.inner_depth = layout->inner_depth;
+        out.rinner = layout->rinner;
+        out.leaves = layout->leaves;
+        layout->depth_consistent = 1;  // written from the tree itself
+        layout->max_inner_depth = (uint32_t)info[1];
+        e = brick_write(b, lean ? BRICK_LEAN : BRICK_LAYOUT, ropes, 0, out, s);
+    } else {
+        if ((r = c->device_alloc(reinterpret_cast<void**>(&out.nodes), n_total * 40, "xn_build_svo: node array")))
+            return r;
+        out.capacity = n_total;
+        e = brick_write(b, BRICK_NODES, ropes, sub ? sub->depth_offset : 0, out, s);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+    if (e != cudaSuccess) {
+        if (layout) layout->release_layout();
+        else c->device_free(out.nodes, n_total * 40);
+        return cuda_fail(e, "xn_build_svo: top-down pass");
+    }
+    if (!layout) {
+        *d_nodes = out.nodes;
+        *d_nodes_bytes = n_total * 40;
+    }
+    stats->total_leaves = stats->unique_leaves = n_leaves;
+    stats->total_nodes = stats->n_nodes = n_total;
+    stats->depth = (Ni ? info[1] + 1 : 0) + (sub ? sub->depth_offset : 0);
+    return XN_OK;
+}
+
 // Builds the reference node array of an RGBA8 grid that is already on the
 // device (packed RGBA, x fastest).  On success *d_nodes is a device buffer of
 // n_nodes*10 words owned by the caller through ctx->device_free.
+//
+// Sparse and rope trees of 16 voxels and more go over bricks (build_bricks).
+// Below that one launch per level over a handful of cells is as quick, and a
+// DAG's hashing needs the cells of every level, with their starts and sizes.
 int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, uint32_t dz, int type, int heuristic,
                      double threshold, uint32_t** d_nodes, uint64_t* d_nodes_bytes, xn_build_stats* stats,
-                     Volume* lean, SubBuild* sub) {
+                     Volume* layout, bool lean, SubBuild* sub) {
     cudaStream_t s = c->stream;
     const uint64_t fit = std::max(ceil_pow2(dx), std::max(ceil_pow2(dy), ceil_pow2(dz)));
     const uint64_t side = sub ? sub->side : fit;
@@ -759,10 +764,13 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
     *d_nodes = nullptr;
     *d_nodes_bytes = 0;
     if (L >= MAX_LEVELS) return fail(XN_ERR_ARG, "xn_build_svo: grid too large");
-    if (sub && (side < fit || (side & (side - 1)) || L == 0 || lean || type != XN_SVO_SPARSE))
+    if (sub && (side < fit || (side & (side - 1)) || L == 0 || layout || type != XN_SVO_SPARSE))
         return fail(XN_ERR_ARG, "xn_build_svo: invalid cube build (side %llu for a %ux%ux%u grid)",
                     (unsigned long long)side, dx, dy, dz);
-    if (lean && L == 0) return LEAN_LEAF_ROOT;
+    if (L >= BRICK_LEVELS && type != XN_SVO_DAG)
+        return build_bricks(c, g, side, L, type == XN_SVO_ROPE_TREE, heuristic, threshold, d_nodes, d_nodes_bytes,
+                            stats, layout, lean, sub);
+    if (layout) return LAYOUT_FROM_NODES;
 
     if (L == 0) {  // a single voxel: the root is a depth-0 leaf
         uint32_t* nodes = nullptr;
@@ -785,20 +793,7 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
     }
 
     std::vector<LevelGeom> geo(L);
-    for (int d = 0; d < L; ++d) {
-        const uint64_t e = side >> d;
-        auto box = [&](uint64_t dim) -> uint32_t {
-            if (d == 0) return 1;
-            uint64_t pe = e * 2;  // parent extent
-            uint64_t m = (dim + pe - 1) / pe;
-            return (uint32_t)std::min<uint64_t>(1ull << d, 2 * m);
-        };
-        geo[d].bx = box(dx);
-        geo[d].by = box(dy);
-        geo[d].bz = box(dz);
-        geo[d].n = (uint64_t)geo[d].bx * geo[d].by * geo[d].bz;
-        geo[d].e = e;
-    }
+    level_boxes(geo.data(), L, side, dx, dy, dz);
 
     Scratch sc(c);
     std::vector<unsigned long long*> size(L), start(L);
@@ -857,7 +852,6 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
         a.stddev = threshold;
         a.ambig_count = counters;
         a.ambig_list = ambig_list;
-        a.lean = lean ? 1 : 0;
         if (heuristic == XN_HEUR_STD_DEV) {
             if ((e = cudaMemsetAsync(counters, 0, 4, s)) != cudaSuccess) break;
             up_level_kernel<XN_HEUR_STD_DEV><<<blocks_for(geo[d].n, T), T, 0, s>>>(a);
@@ -893,70 +887,6 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
     if ((e = cudaMemcpyAsync(&n_total, size[0], 8, cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return cuda_fail(e, "xn_build_svo");
-    if (lean) {
-        if (n_total == 0) return LEAN_LEAF_ROOT;
-        if (n_total >= LEAF) return fail(XN_ERR_FORMAT, "xn_build_svo: more than 2^31 internal nodes");
-        // ---- top-down, lean: the device layout's inner nodes only
-        lean->n_inner = n_total;
-        lean->n_leaves = 0;
-        if ((r = c->device_alloc(reinterpret_cast<void**>(&lean->inner), n_total * 32, "xn_build_svo: inner nodes")) ||
-            (r = c->device_alloc(reinterpret_cast<void**>(&lean->inner_depth), n_total * 4,
-                                 "xn_build_svo: inner depths"))) {
-            lean->release_layout();
-            return r;
-        }
-        for (int d = 0; d < L && e == cudaSuccess; ++d) e = cudaMemsetAsync(start[d], 0xFF, geo[d].n * 8, s);
-        const unsigned long long zero = 0;
-        if (e == cudaSuccess) e = cudaMemcpyAsync(start[0], &zero, 8, cudaMemcpyHostToDevice, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(counters, 0, 16, s);
-        if (e == cudaSuccess) e = cudaMemsetAsync(leaf_count, 0, 8, s);
-        unsigned long long* counts = nullptr;  // [1]: internal nodes written
-        if ((r = sc.alloc(&counts, 2, "xn_build_svo: counters"))) {
-            lean->release_layout();
-            return r;
-        }
-        if (e == cudaSuccess) e = cudaMemsetAsync(counts, 0, 16, s);
-        for (int d = 0; d < L && e == cudaSuccess; ++d) {
-            DownArgs a{};
-            a.g = g;
-            a.cur = geo[d];
-            a.child_is_voxel = d == L - 1;
-            if (d < L - 1) a.child = geo[d + 1];
-            a.depth = d;
-            a.n_total = n_total;
-            a.size = size[d];
-            a.child_size = d < L - 1 ? size[d + 1] : nullptr;
-            a.flags = flags[d];
-            a.child_color = d < L - 1 ? color[d + 1] : nullptr;
-            a.child_flags = d < L - 1 ? flags[d + 1] : nullptr;
-            a.start = start[d];
-            a.child_start = d < L - 1 ? start[d + 1] : nullptr;
-            a.leaves = leaf_count;
-            a.max_depth = counters + 1;
-            a.existing = counts;
-            lean_down_kernel<<<blocks_for(geo[d].n, T), T, 0, s>>>(a, lean->inner, lean->inner_depth);
-            e = cudaGetLastError();
-        }
-        unsigned long long leaves = 0, hcounts[2] = {0, 0};
-        unsigned int hc[2] = {0, 0};
-        if (e == cudaSuccess) e = cudaMemcpyAsync(&leaves, leaf_count, 8, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hc, counters, 8, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(hcounts, counts, 16, cudaMemcpyDeviceToHost, s);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-        if (e == cudaSuccess && hcounts[1] != n_total) {
-            lean->release_layout();
-            return fail(XN_ERR_STATE, "xn_build_svo: %llu of %llu internal nodes written",
-                        (unsigned long long)hcounts[1], (unsigned long long)n_total);
-        }
-        if (e != cudaSuccess) {
-            lean->release_layout();
-            return cuda_fail(e, "xn_build_svo: top-down pass");
-        }
-        stats->total_leaves = stats->unique_leaves = leaves;
-        stats->total_nodes = stats->n_nodes = n_total + leaves;
-        stats->depth = hc[1];
-        return XN_OK;
-    }
     if (n_total > 0xFFFFFFFFull)
         return fail(XN_ERR_FORMAT, "xn_build_svo: %llu nodes exceed the 32-bit node indices of the SVO format",
                     (unsigned long long)n_total);
@@ -1225,52 +1155,41 @@ XN_API int xn_build_svo_volume(xn_ctx* h, const void* d_rgba, uint32_t dx, uint3
     } staged_guard{c, staged, grid_bytes};
     uint32_t* d_nodes = nullptr;
     uint64_t nbytes = 0;
-    if (lean) {
-        // straight into the device layout: no reference nodes, no rope records
-        Volume* v = new (std::nothrow) Volume();
-        if (!v) return fail(XN_ERR_NOMEM, "xn_build_svo_volume: out of host memory");
-        v->ctx = c;
-        r = build_svo_device(c, d_vox, dx, dy, dz, type, heuristic, threshold, &d_nodes, &nbytes, stats, v);
-        if (r == XN_OK) {
-            v->kind = XN_VOLUME_SVO;
-            v->side = stats->side;
-            v->n_nodes = stats->n_nodes;
-            const uint64_t sd = stats->side > 0xFFFFFFFFull ? 0xFFFFFFFFull : stats->side;
-            v->dim[0] = v->dim[1] = v->dim[2] = (uint32_t)sd;
-            v->layout = XN_LAYOUT_COMPACT;
-            v->depth_consistent = 1;  // written from the tree itself
-            if ((r = measure_inner_depth(c, v))) {
-                v->release_layout();
-                delete v;
-                return r;
-            }
-            *out = reinterpret_cast<xn_volume*>(v);
-            return XN_OK;
-        }
-        delete v;
-        if (r != LEAN_LEAF_ROOT) return r;
-        // the root is a leaf: the one-node tree keeps the reference layout
-    }
-    r = build_svo_device(c, d_vox, dx, dy, dz, type, heuristic, threshold, &d_nodes, &nbytes, stats);
-    if (r) return r;
     Volume* v = new (std::nothrow) Volume();
-    if (!v) {
-        c->device_free(d_nodes, nbytes);
-        return fail(XN_ERR_NOMEM, "xn_build_svo_volume: out of host memory");
-    }
+    if (!v) return fail(XN_ERR_NOMEM, "xn_build_svo_volume: out of host memory");
     v->ctx = c;
     v->kind = XN_VOLUME_SVO;
+    // straight into the device layout where that can be, else (a leaf root, a
+    // DAG, a tiny grid) through the node array
+    r = build_svo_device(c, d_vox, dx, dy, dz, type, heuristic, threshold, &d_nodes, &nbytes, stats, v, lean, nullptr);
+    const bool direct = r == XN_OK;
+    if (r == LEAN_LEAF_ROOT || r == LAYOUT_FROM_NODES)
+        r = build_svo_device(c, d_vox, dx, dy, dz, type, heuristic, threshold, &d_nodes, &nbytes, stats);
+    if (r) {
+        delete v;
+        return r;
+    }
     v->side = stats->side;
     v->n_nodes = stats->n_nodes;
     const uint64_t sd = stats->side > 0xFFFFFFFFull ? 0xFFFFFFFFull : stats->side;
     v->dim[0] = v->dim[1] = v->dim[2] = (uint32_t)sd;
-    v->data = d_nodes;
-    v->bytes = nbytes;
     v->has_ropes = type == XN_SVO_ROPE_TREE;
-    if ((r = build_svo_layout(c, v))) {
-        c->device_free(v->data, v->bytes);
-        delete v;
-        return r;
+    if (direct) {
+        v->layout = XN_LAYOUT_COMPACT;
+    } else {
+        v->data = d_nodes;
+        v->bytes = nbytes;
+        if ((r = build_svo_layout(c, v))) {
+            c->device_free(v->data, v->bytes);
+            delete v;
+            return r;
+        }
+        if (lean && v->layout == XN_LAYOUT_COMPACT) {  // no rope records in a lean volume
+            c->device_free(v->rinner, v->n_inner * 32);
+            c->device_free(v->leaves, v->n_leaves * 32);
+            v->rinner = v->leaves = nullptr;
+            v->n_leaves = 0;
+        }
     }
     *out = reinterpret_cast<xn_volume*>(v);
     return XN_OK;
@@ -1464,7 +1383,7 @@ XN_API int xn_build_svo_streamed(xn_ctx* h, uint32_t dx, uint32_t dy, uint32_t d
         uint32_t* d_nodes = nullptr;
         uint64_t nbytes = 0;
         r = build_svo_device(c, d_vox, sx, sy, sz, XN_SVO_SPARSE, heuristic, threshold, &d_nodes, &nbytes, &st, nullptr,
-                             &sub);
+                             false, &sub);
         c->device_free(d_vox, nvox * 4);
         if (r) return r;
         const uint64_t n = st.n_nodes;
@@ -1768,19 +1687,7 @@ int build_static(const uint32_t* d_vox, uint32_t dx, uint32_t dy, uint32_t dz, i
         return e == cudaSuccess ? XN_OK : cuda_fail(e, "xn_build_svo_static");
     }
     LevelGeom geo[MAX_LEVELS];
-    for (int d = 0; d < L; ++d) {
-        const uint64_t e = side >> d;
-        auto box = [&](uint64_t dim) -> uint32_t {
-            if (d == 0) return 1;
-            const uint64_t pe = e * 2;
-            return (uint32_t)std::min<uint64_t>(1ull << d, 2 * ((dim + pe - 1) / pe));
-        };
-        geo[d].bx = box(dx);
-        geo[d].by = box(dy);
-        geo[d].bz = box(dz);
-        geo[d].n = (uint64_t)geo[d].bx * geo[d].by * geo[d].bz;
-        geo[d].e = e;
-    }
+    level_boxes(geo, L, side, dx, dy, dz);
     // size check before anything touches the device
     StaticLevels p{};
     Arena measure{nullptr, ~0ull};
@@ -1793,10 +1700,43 @@ int build_static(const uint32_t* d_vox, uint32_t dx, uint32_t dy, uint32_t dz, i
     void* base = nullptr;
     int r = static_scratch_address(&base);
     if (r) return r;
+    cudaError_t e = cudaSuccess;
+    if (L >= BRICK_LEVELS && type != XN_SVO_DAG) {
+        // over bricks, as xn_build_svo does, with the tree written before the
+        // host knows its size: the kernels leave a node buffer that is too
+        // small alone.  Bricks need a fraction of the scratch that the check
+        // above admits grids by.
+        BrickBuild b{};
+        b.g = g;
+        b.L = L;
+        b.heuristic = heuristic;
+        b.chan_diff = (uint32_t)(uint8_t)threshold;
+        b.stddev = threshold;
+        if (brick_plan(b, side, nullptr) > XN_STATIC_SCRATCH_BYTES)
+            return fail(XN_ERR_BUDGET, "xn_build_svo_static: a %ux%ux%u grid needs more than the static scratch", dx, dy,
+                        dz);
+        brick_plan(b, side, static_cast<unsigned char*>(base));
+        BrickOut out{};
+        out.nodes = d_nodes;
+        out.capacity = capacity;
+        unsigned long long info[2] = {0, 0};
+        e = brick_scan(b, s);
+        if (e == cudaSuccess) e = brick_write(b, BRICK_NODES, type == XN_SVO_ROPE_TREE, 0, out, s);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(info, b.info, sizeof info, cudaMemcpyDeviceToHost, s);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+        if (e != cudaSuccess) return cuda_fail(e, "xn_build_svo_static: build");
+        stats->n_nodes = 8 * info[0] + 1;
+        if (stats->n_nodes > capacity)
+            return fail(XN_ERR_ARG, "xn_build_svo_static: the octree has %llu nodes; the node buffer holds %llu",
+                        (unsigned long long)stats->n_nodes, (unsigned long long)capacity);
+        stats->total_leaves = stats->unique_leaves = 7 * info[0] + 1;
+        stats->total_nodes = stats->n_nodes;
+        stats->depth = info[0] ? info[1] + 1 : 0;
+        return XN_OK;
+    }
     Arena a{static_cast<unsigned char*>(base), XN_STATIC_SCRATCH_BYTES};
     plan_levels(a, p, geo, L, heuristic);
 
-    cudaError_t e = cudaSuccess;
     const unsigned T = 256;
     for (int d = L - 1; d >= 0 && e == cudaSuccess; --d) {
         UpArgs u{};

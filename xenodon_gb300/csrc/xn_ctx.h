@@ -93,11 +93,13 @@ int measure_inner_depth(Ctx* c, Volume* v);
 // depth_consistent flag (volume_io.cu).
 int validate_compact_layout(Ctx* c, Volume* v, const char* what);
 
-// Octree build on the device (svo_build.cu).  With lean == nullptr: the
-// reference node array in *d_nodes.  With lean: only the device layout's
-// inner / inner_depth arrays, written into *lean (sparse trees; no rope
-// records); returns LEAN_LEAF_ROOT when the root is a leaf (no internal nodes).
+// Octree build on the device (svo_build.cu).  With layout == nullptr: the
+// reference node array in *d_nodes.  With layout: the device layout's arrays,
+// written into *layout (lean: only inner / inner_depth, no rope records); that
+// form returns LEAN_LEAF_ROOT when the root is a leaf (no internal nodes) and
+// LAYOUT_FROM_NODES when this tree is only built as a node array.
 constexpr int LEAN_LEAF_ROOT = 1;
+constexpr int LAYOUT_FROM_NODES = 2;
 // A build of one cube of a larger tree (the streamed convert): the cube's
 // side (a power of two at least the grid's dims, where the grid is the part of
 // the whole grid inside the cube), the depth of its root in the whole tree,
@@ -110,7 +112,7 @@ struct SubBuild {
 };
 int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, uint32_t dz, int type, int heuristic,
                      double threshold, uint32_t** d_nodes, uint64_t* d_nodes_bytes, xn_build_stats* stats,
-                     Volume* lean = nullptr, SubBuild* sub = nullptr);
+                     Volume* layout = nullptr, bool lean = false, SubBuild* sub = nullptr);
 
 int fail(int code, const char* fmt, ...) __attribute__((format(printf, 2, 3)));
 int cuda_fail(cudaError_t e, const char* what);
