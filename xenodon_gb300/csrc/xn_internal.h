@@ -51,6 +51,7 @@ struct RenderLaunch {
     int shared_stacks;            // esvo and masked svo-df with their stacks in shared memory
     int naive_resume;             // svo-naive's find resumes from the previous step's path
     int df_packet;                // masked svo-df walked by the whole warp (df_packet_kernel)
+    int df_steps;                 // masked svo-df one ray per lane, every step alike (df_steps_kernel)
     float df_lane_side;           // child size of the nodes below which the lanes walk alone: 2^-D
                                   // (one level; D the deepest internal node's depth) or 2^-(D-1)
                                   // (two levels), or 0
@@ -85,6 +86,7 @@ struct alignas(16) BatchJob {
     int32_t tex_normalized;
     int32_t depth_consistent;
     int32_t form;  // XN_BATCH_* form of this job (batch_spec)
+    int32_t df_steps;    // svo-df: one ray per lane (trace_df_steps)
     float df_lane_side;  // svo-df: child size 2^-D of the nodes whose children the lanes walk alone, or 0
     unsigned long long tex;
     const void* grid;
@@ -107,7 +109,7 @@ BatchJob make_batch_job(const RenderLaunch& L);
 // Batch kernel forms: one traversal (and layout) inlined when every job of
 // the batch shares it, else the generic per-pixel dispatch.
 enum { XN_BATCH_ANY = 0, XN_BATCH_DDA_TEX_NORM, XN_BATCH_DDA_TEX_RAW, XN_BATCH_ESVO, XN_BATCH_NAIVE, XN_BATCH_DF,
-       XN_BATCH_ROPE, XN_BATCH_FORMS };
+       XN_BATCH_ROPE, XN_BATCH_DF_STEPS, XN_BATCH_FORMS };
 // The form a job needs (XN_BATCH_*).
 int batch_spec(const BatchJob& j);
 // Launches the persistent kernel over a job table already in device memory
