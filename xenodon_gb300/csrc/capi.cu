@@ -529,6 +529,7 @@ int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_p
         L.inner_depth = v->inner_depth;
         L.leaves = v->leaves;
         L.depth_consistent = v->depth_consistent;
+        L.shallow = v->depth_consistent && v->max_inner_depth < (uint32_t)XN_SHALLOW_DEPTH;
         if (traversal == XN_TRAV_SVO_ROPE && v->layout == XN_LAYOUT_COMPACT && !v->rinner)
             return fail(XN_ERR_ARG, "svo-rope: the octree was built lean, without rope records");
         // traversal stacks: esvo's in shared memory, svo-df's in local memory

@@ -25,6 +25,7 @@ constexpr uint32_t DEPTH_MASK = 0x7FFFFFFFu;
 constexpr uint32_t SVO_MAX_ITER = 1u << 22;
 constexpr int FIND_MAX_DEPTH = 64;
 constexpr int STACK_DEPTH = 23;  // FLOAT_MANTISSA_BITS, resources/common.glsl:37
+constexpr int SHALLOW_ROWS = XN_SHALLOW_DEPTH;
 
 struct Outputs {
     uint32_t* rgba;      // packed RGBA8, row pitch out_w
@@ -377,13 +378,21 @@ constexpr int FIX_BITS = 30;
 constexpr int FIX_DEPTH = 24;
 
 struct LocalPath {
+    static constexpr bool DEEP = true;
     uint32_t n[FIX_DEPTH];
     __device__ __forceinline__ uint32_t& node(int level) { return n[level - 1]; }
 };
 struct SharedPath {
+    static constexpr bool DEEP = true;
     uint32_t* base;  // this thread's column
     uint32_t stride;
     __device__ __forceinline__ uint32_t& node(int level) { return base[(level - 1) * stride]; }
+};
+template <int STRIDE>
+struct ShallowPath {  // octrees of depth <= SHALLOW_ROWS (leaves at most that deep)
+    static constexpr bool DEEP = false;
+    uint32_t* base;  // this thread's column
+    __device__ __forceinline__ uint32_t& node(int level) { return base[(level - 1) * STRIDE]; }
 };
 struct FindPath {
     int depth = -1;          // depth of the last leaf found, -1: none (or too deep to cache)
@@ -408,6 +417,8 @@ __device__ __forceinline__ uint32_t fix_coord(float p) {
 
 __device__ __forceinline__ float fix_to_float(uint32_t v) { return (float)v * (1.0f / 1073741824.0f); }
 
+// Path::DEEP false (octrees of depth <= SHALLOW_ROWS): every node is within
+// the path, so the descent ends at a leaf by itself.
 template <bool COUNT, class Acc, class Path>
 __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Path& pn, V3 pos, V3& base,
                                                 float& side, uint32_t& loads, uint32_t& err) {
@@ -427,7 +438,7 @@ __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Pa
     }
     // the path's levels up to the resumed one are already in place
     for (;; ++level) {
-        if (a.is_leaf(index) || level == FIX_DEPTH) break;
+        if (a.is_leaf(index) || (Path::DEEP && level == FIX_DEPTH)) break;
         const int b = FIX_BITS - 1 - level;
         const uint32_t k = (((px >> b) & 1u) << 2) | (((py >> b) & 1u) << 1) | ((pz >> b) & 1u);
         index = a.child(index, k);
@@ -436,7 +447,7 @@ __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Pa
     const uint32_t keep = ~((1u << (FIX_BITS - level)) - 1u);
     V3 offset = v3(fix_to_float(px & keep), fix_to_float(py & keep), fix_to_float(pz & keep));
     float extent = __uint_as_float((uint32_t)(127 - level) << 23);  // 2^-level
-    if (!a.is_leaf(index)) {
+    if (Path::DEEP && !a.is_leaf(index)) {
         // below depth 24 (deeper than any grid of 2^24 voxels per axis): the
         // reference's float descent
         for (;; ++level) {
@@ -458,7 +469,7 @@ __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Pa
     base = offset;
     side = extent;
     if (COUNT) loads += 2u * (uint32_t)level + 1u;
-    if (level <= FIX_DEPTH) {
+    if (!Path::DEEP || level <= FIX_DEPTH) {
         path.depth = level;
         path.cx = px & keep;
         path.cy = py & keep;
@@ -583,6 +594,7 @@ __device__ V3 trace_df(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& er
 // shared memory with one column per thread (entry i of a thread at i * stride
 // from its column start, so a warp touching one entry hits 32 banks).
 struct LocalStacks {
+    static constexpr bool T_MAX = true;
     uint32_t a[STACK_DEPTH];
     uint32_t b[STACK_DEPTH];
     __device__ __forceinline__ uint32_t& first(uint32_t i) { return a[i]; }
@@ -590,11 +602,23 @@ struct LocalStacks {
 };
 
 struct SharedStacks {
+    static constexpr bool T_MAX = true;
     uint32_t* a;  // this thread's column in each array
     uint32_t* b;
     uint32_t stride;
     __device__ __forceinline__ uint32_t& first(uint32_t i) { return a[i * stride]; }
     __device__ __forceinline__ uint32_t& second(uint32_t i) { return b[i * stride]; }
+};
+
+// esvo's parents alone, for octrees whose internal nodes are at most
+// SHALLOW_ROWS - 1 deep: scales STACK_DEPTH - 1 down to STACK_DEPTH -
+// SHALLOW_ROWS, one column of shared memory per thread.
+template <int STRIDE>
+struct NodeStack {
+    static constexpr bool T_MAX = false;
+    uint32_t* a;  // this thread's column
+    __device__ __forceinline__ uint32_t& first(uint32_t i) { return a[(i - (STACK_DEPTH - SHALLOW_ROWS)) * STRIDE]; }
+    __device__ __forceinline__ uint32_t& second(uint32_t i) { return first(i); }
 };
 
 // resources/svo_df.comp:6-67 for octrees whose depth fields match the tree
@@ -746,13 +770,26 @@ __device__ __forceinline__ uint32_t cxor(uint32_t x, bool ax, bool ay, bool az) 
 // resources/esvo.comp:30-136
 // ESVO's (parent, t_max) stack, indexed by scale: LocalStacks / SharedStacks
 // (t_max kept as its bits).
+//
+// Stacks::T_MAX false (NodeStack, octrees of depth <= SHALLOW_ROWS): only the
+// parents are stacked.  The reference's t_max is the least exit t of the
+// ancestors and the ray's own limit; a child's corner is no farther than its
+// parent's on any axis and the rounded t of a plane is monotonic in its
+// position, so the child's own tc_max is no larger than any ancestor's, and
+// tv_max = min(t_max, tc_max) = min(limit, tc_max).  And planes that are 2^-12
+// or more apart have different t's (|t_coeff| 2^-12 is far above the rounding
+// of pos * t_coeff), so tc_max == h only where the child leaves through its
+// parent's exit plane: a parent that was not stacked is never popped, and the
+// stack needs no initial value.
 template <bool COUNT, class Acc, class Stacks = LocalStacks>
 __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& err, Stacks* shared_stacks = nullptr) {
     const uint32_t depth = STACK_DEPTH;
     Stacks local;
     Stacks& stk = shared_stacks ? *shared_stacks : local;  // first: parent, second: t_max bits
+    if constexpr (Stacks::T_MAX) {
 #pragma unroll
-    for (int i = 0; i < STACK_DEPTH; ++i) { stk.first(i) = 0; stk.second(i) = 0u; }
+        for (int i = 0; i < STACK_DEPTH; ++i) { stk.first(i) = 0; stk.second(i) = 0u; }
+    }
 
     V3 t_coeff = v3(1.0f / -fabsf(rd.x), 1.0f / -fabsf(rd.y), 1.0f / -fabsf(rd.z));
     V3 t_bias = t_coeff * ro;
@@ -804,7 +841,7 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
             } else {
                 if (tc_max < h) {
                     stk.first(scale) = parent;
-                    stk.second(scale) = __float_as_uint(t_max);
+                    if constexpr (Stacks::T_MAX) stk.second(scale) = __float_as_uint(t_max);
                 }
                 h = tc_max;
                 parent = child;
@@ -820,7 +857,7 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
                 if (ax) pos.x = pos.x + scale_exp2;
                 if (ay) pos.y = pos.y + scale_exp2;
                 if (az) pos.z = pos.z + scale_exp2;
-                t_max = tv_max;
+                if constexpr (Stacks::T_MAX) t_max = tv_max;
                 continue;
             }
         }
@@ -843,7 +880,7 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
             if (scale >= depth) break;  // the loop condition ends the ray
             scale_exp2 = __uint_as_float((scale - depth + 127u) << 23);
             parent = stk.first(scale);
-            t_max = __uint_as_float(stk.second(scale));
+            if constexpr (Stacks::T_MAX) t_max = __uint_as_float(stk.second(scale));
             uint32_t shx = __float_as_uint(pos.x) >> scale;
             uint32_t shy = __float_as_uint(pos.y) >> scale;
             uint32_t shz = __float_as_uint(pos.z) >> scale;
@@ -1105,6 +1142,10 @@ __device__ __forceinline__ void svo_pixel(const Frame& f, const Acc& a, const Ou
         __shared__ uint32_t s_path[FIX_DEPTH * BLOCK_THREADS];
         SharedPath sp{s_path + threadIdx.x, BLOCK_THREADS};
         total = trace_naive<COUNT, Acc, true, SharedPath>(a, f.translation, rd, loads, err, &sp);
+    } else if constexpr (TRAV == XN_TRAV_SVO_NAIVE_SHALLOW) {
+        __shared__ uint32_t s_path[SHALLOW_ROWS * BLOCK_THREADS];
+        ShallowPath<BLOCK_THREADS> sp{s_path + threadIdx.x};
+        total = trace_naive<COUNT, Acc, true, ShallowPath<BLOCK_THREADS>>(a, f.translation, rd, loads, err, &sp);
     } else if (TRAV == XN_TRAV_SVO_NAIVE_ROOT) {
         total = trace_naive<COUNT, Acc, false>(a, f.translation, rd, loads, err);
     } else if (TRAV == XN_TRAV_SVO_DF) {
@@ -1526,6 +1567,23 @@ __global__ void __launch_bounds__(SHARED_BLOCK) shared_stack_kernel(Frame f, Acc
     write_outputs(f, o, ix, iy, total * voxel_emission_coeff(f, rd), loads, err);
 }
 
+template <bool COUNT>
+__global__ void __launch_bounds__(SHARED_BLOCK) esvo_shallow_kernel(Frame f, CompactNodes a, Outputs o) {
+    __shared__ uint32_t s_a[SHALLOW_ROWS * SHARED_BLOCK];
+    fill_unorm_lut();
+    uint32_t ix, iy;
+    if (!pixel_of_thread_bt<SHARED_BLOCK>(f, ix, iy)) return;
+    NodeStack<SHARED_BLOCK> stk{s_a + threadIdx.x};
+    const V3 rd = primary_ray(f, ix, iy);
+    uint32_t loads = 0, err = 0;
+    // resources/esvo.comp:148-152
+    V3 ro = f.translation + vs(1.0f);
+    const float t0 = aabb_entry(vs(1.0f), vs(2.0f), ro, rd);
+    ro = ro + rd * fmaxf(t0, 0.0f);
+    const V3 total = trace_esvo<COUNT, CompactNodes, NodeStack<SHARED_BLOCK>>(a, ro, rd, loads, err, &stk);
+    write_outputs(f, o, ix, iy, total * voxel_emission_coeff(f, rd), loads, err);
+}
+
 template <int TRAV, class Acc>
 static void launch_svo_any(bool count, const Frame& f, const Acc& a, const Outputs& o, dim3 grid, cudaStream_t s) {
     if constexpr (TRAV == XN_TRAV_SVO_ROPE) {
@@ -1542,6 +1600,7 @@ static void launch_traversal(int traversal, bool count, const Frame& f, const Ac
                              cudaStream_t s) {
     switch (traversal) {
     case XN_TRAV_SVO_NAIVE: launch_svo_any<XN_TRAV_SVO_NAIVE>(count, f, a, o, grid, s); break;
+    case XN_TRAV_SVO_NAIVE_SHALLOW: launch_svo_any<XN_TRAV_SVO_NAIVE_SHALLOW>(count, f, a, o, grid, s); break;
     case XN_TRAV_SVO_NAIVE_ROOT: launch_svo_any<XN_TRAV_SVO_NAIVE_ROOT>(count, f, a, o, grid, s); break;
     case XN_TRAV_ESVO: launch_svo_any<XN_TRAV_ESVO>(count, f, a, o, grid, s); break;
     case XN_TRAV_SVO_DF: launch_svo_any<XN_TRAV_SVO_DF>(count, f, a, o, grid, s); break;
@@ -1623,7 +1682,9 @@ cudaError_t launch_render(const RenderLaunch& L, cudaStream_t stream) {
             else shared_stack_kernel<XN_TRAV_ESVO, false><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
         } else {
             const CompactNodes acc{L.inner, L.inner_depth};
-            if (count) shared_stack_kernel<XN_TRAV_ESVO, true><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
+            if (L.shallow && count) esvo_shallow_kernel<true><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
+            else if (L.shallow) esvo_shallow_kernel<false><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
+            else if (count) shared_stack_kernel<XN_TRAV_ESVO, true><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
             else shared_stack_kernel<XN_TRAV_ESVO, false><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
         }
     } else if (L.traversal == XN_TRAV_SVO_DF && L.df_steps && !L.shared_stacks && L.layout == XN_LAYOUT_COMPACT &&
@@ -1652,7 +1713,8 @@ cudaError_t launch_render(const RenderLaunch& L, cudaStream_t stream) {
         launch_traversal(L.traversal, count, f, RopeNodes{L.rinner, L.inner_depth, L.leaves}, o, grid, stream);
     } else {
         int trav = L.traversal == XN_TRAV_SVO_DF && L.depth_consistent ? XN_TRAV_SVO_DF_MASKED : L.traversal;
-        if (trav == XN_TRAV_SVO_NAIVE && !L.naive_resume) trav = XN_TRAV_SVO_NAIVE_ROOT;
+        if (trav == XN_TRAV_SVO_NAIVE)
+            trav = !L.naive_resume ? XN_TRAV_SVO_NAIVE_ROOT : L.shallow ? XN_TRAV_SVO_NAIVE_SHALLOW : trav;
         launch_traversal(trav, count, f, CompactNodes{L.inner, L.inner_depth}, o, grid, stream);
     }
     return cudaGetLastError();

@@ -18,8 +18,12 @@ enum {
     XN_TRAV_SVO_DF = 3,
     XN_TRAV_SVO_ROPE = 4,
     XN_TRAV_SVO_DF_MASKED = 5,  // svo-df on an octree with consistent depth fields (render.cu)
-    XN_TRAV_SVO_NAIVE_ROOT = 6  // svo-naive with every find from the root
+    XN_TRAV_SVO_NAIVE_ROOT = 6,  // svo-naive with every find from the root
+    XN_TRAV_SVO_NAIVE_SHALLOW = 7  // svo-naive on an octree of depth <= XN_SHALLOW_DEPTH
 };
+// Depth up to which octrees (grids of up to 4096 voxels a side) get the forms
+// of esvo and svo-naive with fewer rows of stack or path per thread.
+constexpr int XN_SHALLOW_DEPTH = 12;
 
 // Everything one traversal launch needs; built by the C-ABI layer from an
 // xn_camera + xn_params + volume.
@@ -49,6 +53,7 @@ struct RenderLaunch {
     const uint32_t* leaves;
     int depth_consistent;         // every internal node's depth field = its depth in the tree
     int shared_stacks;            // esvo and masked svo-df with their stacks in shared memory
+    int shallow;                  // depth consistent, and no leaf deeper than XN_SHALLOW_DEPTH
     int naive_resume;             // svo-naive's find resumes from the previous step's path
     int df_packet;                // masked svo-df walked by the whole warp (df_packet_kernel)
     int df_steps;                 // masked svo-df one ray per lane, every step alike (df_steps_kernel)
