@@ -34,10 +34,13 @@
 #include "../../include/xenodon.h"
 #include "xn_bricks.h"
 #include "xn_ctx.h"
+#include "xn_heuristics.cuh"
 #include "xn_internal.h"
 
 namespace xn {
 namespace {
+
+using namespace heur;
 
 constexpr uint32_t LEAF = 0x80000000u;
 constexpr unsigned long long NONE = ~0ull;
@@ -116,48 +119,6 @@ __device__ __forceinline__ uint64_t index_of(const LevelGeom& L, uint32_t x, uin
 
 __device__ __forceinline__ uint32_t digit_sum(uint32_t x, uint32_t y, uint32_t z) {
     return 4u * __popc(x) + 2u * __popc(y) + __popc(z);
-}
-
-__device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
-
-__device__ __forceinline__ uint64_t clamped_count(const GridDev& g, uint64_t ox, uint64_t oy, uint64_t oz, uint64_t e) {
-    return (umin64(g.dx, ox + e) - ox) * (umin64(g.dy, oy + e) - oy) * (umin64(g.dz, oz + e) - oz);
-}
-
-// ------------------------------------------------------------- heuristics ---
-
-// Grid::stddev_scan (Grid.cpp:139-214) run literally, the sequential double
-// loop in z, y, x order, over the cell's part of the grid.
-__device__ __noinline__ bool sequential_split(const GridDev& g, uint64_t x0, uint64_t y0, uint64_t z0, uint64_t e,
-                                              const unsigned long long* s1, double threshold) {
-    const uint64_t x1 = umin64(g.dx, x0 + e), y1 = umin64(g.dy, y0 + e), z1 = umin64(g.dz, z0 + e);
-    const double nd = (double)((x1 - x0) * (y1 - y0) * (z1 - z0));
-    double avg[4];
-    for (int c = 0; c < 4; ++c) avg[c] = (double)s1[c] / nd;
-    double s = 0.0;
-    for (uint64_t z = z0; z < z1; ++z)
-        for (uint64_t y = y0; y < y1; ++y)
-            for (uint64_t x = x0; x < x1; ++x) {
-                const uint32_t v = __ldg(g.vox + x + (uint64_t)g.dx * (y + (uint64_t)g.dy * z));
-                const double d0 = (double)(v & 0xFFu) - avg[0];
-                const double d1 = (double)((v >> 8) & 0xFFu) - avg[1];
-                const double d2 = (double)((v >> 16) & 0xFFu) - avg[2];
-                const double d3 = (double)(v >> 24) - avg[3];
-                s += ((d0 * d0 + d1 * d1) + d2 * d2) + d3 * d3;
-            }
-    return sqrt(s / nd) > threshold;
-}
-
-// Whether the standard deviation sqrt(E)/n, E = n sum(x^2) - sum(x)^2 exact,
-// is above the threshold, as the reference's sequential double sum decides:
-// that sum differs from the exact value by at most (n + 16) 2^-52 relative,
-// and inside that band its own loop decides (seq).
-__device__ bool stddev_split(double E, uint64_t n, double threshold, bool& seq) {
-    const double nd = (double)n;
-    const double sd = sqrt(E / (nd * nd));
-    const double band = (nd + 16.0) * 2.220446049250313e-16 * sd + 1e-300;
-    seq = fabs(sd - threshold) <= band;
-    return sd > threshold;
 }
 
 // Statistics of a cell inside a brick.  Channels 0 and 2, and 1 and 3, share a

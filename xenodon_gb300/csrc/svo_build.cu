@@ -41,34 +41,26 @@
 #include "../../include/xenodon.h"
 #include "xn_bricks.h"
 #include "xn_ctx.h"
+#include "xn_heuristics.cuh"
 #include "xn_internal.h"
 #include "xn_scan.cuh"
 
 namespace xn {
 namespace {
 
+using namespace heur;
 using namespace scan;
 
 constexpr uint32_t LEAF = 0x80000000u;
 constexpr uint64_t NONE = ~0ull;
-constexpr uint8_t F_LEAF = 1, F_INSIDE = 2, F_AMBIG = 4;
+constexpr uint8_t F_LEAF = 1, F_INSIDE = 2;
 
 __device__ __forceinline__ uint32_t vox_at(const GridDev& g, uint32_t x, uint32_t y, uint32_t z) {
     return __ldg(g.vox + (uint64_t)x + (uint64_t)g.dx * ((uint64_t)y + (uint64_t)g.dy * z));
 }
 
-__device__ __forceinline__ uint64_t umin64(uint64_t a, uint64_t b) { return a < b ? a : b; }
-
 __device__ __forceinline__ uint32_t byte_min4(uint32_t a, uint32_t b) { return __vminu4(a, b); }
 __device__ __forceinline__ uint32_t byte_max4(uint32_t a, uint32_t b) { return __vmaxu4(a, b); }
-
-// Voxels of the cell clamped to the grid (Grid::vol_scan's bmin/bmax clamp).
-__device__ __forceinline__ uint64_t clamped_count(const GridDev& g, uint64_t ox, uint64_t oy, uint64_t oz, uint64_t e) {
-    uint64_t nx = umin64(g.dx, ox + e) - ox;
-    uint64_t ny = umin64(g.dy, oy + e) - oy;
-    uint64_t nz = umin64(g.dz, oz + e) - oz;
-    return nx * ny * nz;
-}
 
 struct UpArgs {
     GridDev g;
@@ -82,8 +74,7 @@ struct UpArgs {
     uint8_t* flags;
     uint32_t chan_diff;     // ChannelDiff threshold (0..255)
     double stddev;          // StdDev threshold
-    unsigned int* ambig_count;
-    unsigned long long* ambig_list;
+    int sequential;         // StdDev: every decision through the reference's loop (a check mode)
 };
 
 __device__ __forceinline__ void cell_coords(uint64_t i, const LevelGeom& L, uint32_t& x, uint32_t& y, uint32_t& z) {
@@ -158,7 +149,6 @@ __global__ void up_level_kernel(UpArgs a) {
     const uint64_t n = clamped_count(a.g, ox, oy, oz, e);
     uint32_t avg = 0;
     bool split;
-    bool ambiguous = false;
     if (HEUR == XN_HEUR_CHANNEL_DIFF) {
         CDStats& out = static_cast<CDStats*>(a.stats)[i];
 #pragma unroll
@@ -183,82 +173,18 @@ __global__ void up_level_kernel(UpArgs a) {
             avg |= (uint32_t)(uint8_t)((double)s[c] / nd) << (8 * c);  // Grid.cpp:180-186,208-212
             E += (unsigned __int128)n * q[c] - (unsigned __int128)s[c] * s[c];
         }
-        if (E == 0) {
-            split = 0.0 > a.stddev;  // every voxel equals the mean: the double sum is exactly 0
-        } else {
-            // sqrt(sum/n) computed exactly up to double rounding; the
-            // reference's sequential double sum differs from the exact value
-            // by at most (n + 16) * 2^-52 relative; inside that band the
-            // decision is taken from the reference's own loop (stddev_fixup).
-            double var = (double)E / (nd * nd);
-            double sd = sqrt(var);
-            double band = (nd + 16.0) * 2.220446049250313e-16 * sd + 1e-300;
-            if (fabs(sd - a.stddev) <= band) ambiguous = true;
-            split = sd > a.stddev;
-        }
+        bool seq = false;
+        split = E == 0 ? 0.0 > a.stddev : stddev_split((double)E, n, a.stddev, seq);
+        if (seq || a.sequential) split = sequential_split(a.g, ox, oy, oz, e, s, a.stddev);
     }
     a.color[i] = avg;
-    if (ambiguous) {
-        unsigned int slot = atomicAdd(a.ambig_count, 1u);
-        a.ambig_list[slot] = i;
-    }
     const bool leaf = (!split && fully) || e == 1;
-    a.flags[i] = (leaf ? F_LEAF : 0) | F_INSIDE | (ambiguous ? F_AMBIG : 0);
+    a.flags[i] = (leaf ? F_LEAF : 0) | F_INSIDE;
     uint64_t sz = 1;
     if (!leaf) {
 #pragma unroll
         for (int k = 0; k < 8; ++k) sz += child_size(a, x, y, z, k);
     }
-    a.size[i] = sz;
-}
-
-// Grid::stddev_scan (Grid.cpp:139-214) run literally -- the sequential double
-// loop in z, y, x order -- for the cells whose decision lies inside the
-// rounding band of the exact computation.
-__global__ void stddev_fixup_kernel(UpArgs a, unsigned int count) {
-    unsigned int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= count) return;
-    uint64_t i = a.ambig_list[j];
-    uint32_t x, y, z;
-    cell_coords(i, a.cur, x, y, z);
-    const uint64_t e = a.cur.e;
-    const uint64_t x0 = x * e, y0 = y * e, z0 = z * e;
-    const uint64_t x1 = umin64(a.g.dx, x0 + e), y1 = umin64(a.g.dy, y0 + e),
-                   z1 = umin64(a.g.dz, z0 + e);
-    const SDStats& st = static_cast<const SDStats*>(a.stats)[i];
-    const uint64_t n = (x1 - x0) * (y1 - y0) * (z1 - z0);
-    const double nd = (double)n;
-    double avg[4];
-    for (int c = 0; c < 4; ++c) avg[c] = (double)st.s1[c] / nd;
-    double s = 0.0;
-    for (uint64_t zz = z0; zz < z1; ++zz)
-        for (uint64_t yy = y0; yy < y1; ++yy)
-            for (uint64_t xx = x0; xx < x1; ++xx) {
-                uint32_t v = vox_at(a.g, (uint32_t)xx, (uint32_t)yy, (uint32_t)zz);
-                double d0 = (double)(v & 0xFFu) - avg[0];
-                double d1 = (double)((v >> 8) & 0xFFu) - avg[1];
-                double d2 = (double)((v >> 16) & 0xFFu) - avg[2];
-                double d3 = (double)(v >> 24) - avg[3];
-                s += ((d0 * d0 + d1 * d1) + d2 * d2) + d3 * d3;
-            }
-    const bool split = sqrt(s / nd) > a.stddev;
-    const bool fully = x0 + e <= a.g.dx && y0 + e <= a.g.dy && z0 + e <= a.g.dz;
-    const bool leaf = (!split && fully) || e == 1;
-    a.flags[i] = (leaf ? F_LEAF : 0) | F_INSIDE;
-}
-
-// Recomputes subtree sizes of a level after stddev_fixup changed decisions.
-__global__ void resize_level_kernel(UpArgs a) {
-    uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= a.cur.n) return;
-    if (a.flags[i] & F_LEAF) {
-        a.size[i] = 1;
-        return;
-    }
-    uint32_t x, y, z;
-    cell_coords(i, a.cur, x, y, z);
-    uint64_t sz = 1;
-    for (int k = 0; k < 8; ++k) sz += child_size(a, x, y, z, k);
     a.size[i] = sz;
 }
 
@@ -541,16 +467,23 @@ __global__ void dag_insert_kernel(DagLevel a, Slot* table, uint64_t mask, unsign
     uint64_t post;
     if (!dag_node(a, id, k, post)) return;
     uint64_t slot = key_hash(k) & mask;
+    // A depth's leaves share a few slots (one per colour): an owner is claimed,
+    // and a class's position lowered, only where a plain read says that it is
+    // still free, or still larger.  (Both only ever change towards claimed and
+    // lower, so an old value costs an atomic and nothing else.)  203x143x197 CT
+    // shell, the voxels' depth: 1977 us with an atomic per node.
     for (uint64_t probe = 0; probe <= mask; ++probe) {
-        unsigned long long o = atomicCAS(&table[slot].owner, NONE, (unsigned long long)id);
-        if (o == NONE) {
-            atomicMin(&table[slot].rep, (unsigned long long)post);
-            return;
+        unsigned long long o = *const_cast<volatile unsigned long long*>(&table[slot].owner);
+        if (o == NONE) o = atomicCAS(&table[slot].owner, NONE, (unsigned long long)id);
+        bool same = o == NONE || o == id;
+        if (!same) {
+            DagKey ko;
+            uint64_t po;
+            same = dag_node(a, o, ko, po) && key_eq(k, ko);
         }
-        DagKey ko;
-        uint64_t po;
-        if (dag_node(a, o, ko, po) && key_eq(k, ko)) {
-            atomicMin(&table[slot].rep, (unsigned long long)post);
+        if (same) {
+            if (*const_cast<volatile unsigned long long*>(&table[slot].rep) > post)
+                atomicMin(&table[slot].rep, (unsigned long long)post);
             return;
         }
         slot = (slot + 1) & mask;
@@ -800,38 +733,37 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
     std::vector<uint32_t*> color(L);
     std::vector<uint8_t*> flags(L);
     int r;
-    for (int d = 0; d < L; ++d) {
-        if ((r = sc.alloc(&size[d], geo[d].n, "xn_build_svo: sizes")) ||
-            (r = sc.alloc(&start[d], geo[d].n, "xn_build_svo: starts")) ||
-            (r = sc.alloc(&color[d], geo[d].n, "xn_build_svo: colours")) ||
-            (r = sc.alloc(&flags[d], geo[d].n, "xn_build_svo: flags")))
-            return r;
-    }
     const uint64_t stat_bytes = heuristic == XN_HEUR_STD_DEV ? sizeof(SDStats) : sizeof(CDStats);
     void* stats_buf[2] = {nullptr, nullptr};
-    {
-        // level d writes buffer d & 1 and reads d + 1's: size each for its own levels
-        uint64_t big[2] = {1, 1};
-        for (int d = 0; d < L; ++d) big[d & 1] = std::max(big[d & 1], geo[d].n);
-        uint8_t* p0 = nullptr;
-        uint8_t* p1 = nullptr;
-        if ((r = sc.alloc(&p0, big[0] * stat_bytes, "xn_build_svo: scan statistics")) ||
-            (r = sc.alloc(&p1, big[1] * stat_bytes, "xn_build_svo: scan statistics")))
-            return r;
-        stats_buf[0] = p0;
-        stats_buf[1] = p1;
-    }
-    unsigned int* counters = nullptr;  // [0] ambiguous count, [1] max depth
+    unsigned int* counters = nullptr;  // [0] hash table overflow, [1] max depth
     unsigned long long* leaf_count = nullptr;
-    unsigned long long* ambig_list = nullptr;
-    if ((r = sc.alloc(&counters, 4, "xn_build_svo: counters")) ||
-        (r = sc.alloc(&leaf_count, 1, "xn_build_svo: counters")))
-        return r;
-    if (heuristic == XN_HEUR_STD_DEV) {
-        uint64_t big = 0;
-        for (int d = 0; d < L; ++d) big = std::max(big, geo[d].n);
-        if ((r = sc.alloc(&ambig_list, big, "xn_build_svo: stddev list"))) return r;
-    }
+    unsigned long long* existing = nullptr;  // per level: existing cells, internal cells
+    // all of it in one allocation: measured, then placed
+    auto plan = [&](unsigned char* base) -> uint64_t {
+        uint64_t used = 0;
+        auto take = [&](uint64_t bytes) -> void* {
+            void* p = base ? base + used : nullptr;
+            used += (bytes + 255) & ~255ull;
+            return p;
+        };
+        uint64_t big2[2] = {1, 1};  // level d writes statistics d & 1 and reads d + 1's
+        for (int d = 0; d < L; ++d) {
+            size[d] = static_cast<unsigned long long*>(take(geo[d].n * 8));
+            start[d] = static_cast<unsigned long long*>(take(geo[d].n * 8));
+            color[d] = static_cast<uint32_t*>(take(geo[d].n * 4));
+            flags[d] = static_cast<uint8_t*>(take(geo[d].n));
+            big2[d & 1] = std::max(big2[d & 1], geo[d].n);
+        }
+        stats_buf[0] = take(big2[0] * stat_bytes);
+        stats_buf[1] = take(big2[1] * stat_bytes);
+        counters = static_cast<unsigned int*>(take(16));
+        leaf_count = static_cast<unsigned long long*>(take(8));
+        existing = static_cast<unsigned long long*>(take(16 * (uint64_t)L));
+        return used;
+    };
+    unsigned char* base = nullptr;
+    if ((r = sc.alloc(&base, plan(nullptr), "xn_build_svo: scratch"))) return r;
+    plan(base);
 
     cudaError_t e = cudaSuccess;
     const unsigned T = 256;
@@ -850,32 +782,10 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
         a.flags = flags[d];
         a.chan_diff = (uint32_t)(uint8_t)threshold;
         a.stddev = threshold;
-        a.ambig_count = counters;
-        a.ambig_list = ambig_list;
-        if (heuristic == XN_HEUR_STD_DEV) {
-            if ((e = cudaMemsetAsync(counters, 0, 4, s)) != cudaSuccess) break;
+        a.sequential = heuristic == XN_HEUR_STD_DEV && getenv("XN_BUILD_STDDEV_SEQUENTIAL") != nullptr;
+        if (heuristic == XN_HEUR_STD_DEV)
             up_level_kernel<XN_HEUR_STD_DEV><<<blocks_for(geo[d].n, T), T, 0, s>>>(a);
-            unsigned int amb = 0;
-            if ((e = cudaMemcpyAsync(&amb, counters, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
-            if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;
-            if (getenv("XN_BUILD_STDDEV_SEQUENTIAL")) {
-                // check mode: every in-grid decision through the reference loop
-                amb = 0;
-                std::vector<uint8_t> hf(geo[d].n);
-                cudaMemcpy(hf.data(), flags[d], geo[d].n, cudaMemcpyDeviceToHost);
-                std::vector<unsigned long long> lst;
-                for (uint64_t i = 0; i < geo[d].n; ++i)
-                    if (hf[i] & F_INSIDE) lst.push_back(i);
-                amb = (unsigned)lst.size();
-                cudaMemcpy(ambig_list, lst.data(), lst.size() * 8, cudaMemcpyHostToDevice);
-            }
-            if (amb) {
-                stddev_fixup_kernel<<<blocks_for(amb, 64), 64, 0, s>>>(a, amb);
-                resize_level_kernel<<<blocks_for(geo[d].n, T), T, 0, s>>>(a);
-            }
-        } else {
-            up_level_kernel<XN_HEUR_CHANNEL_DIFF><<<blocks_for(geo[d].n, T), T, 0, s>>>(a);
-        }
+        else up_level_kernel<XN_HEUR_CHANNEL_DIFF><<<blocks_for(geo[d].n, T), T, 0, s>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
     }
     if (e != cudaSuccess) return cuda_fail(e, "xn_build_svo: bottom-up pass");
@@ -892,8 +802,6 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
                     (unsigned long long)n_total);
 
     const bool dag = type == XN_SVO_DAG;
-    unsigned long long* existing = nullptr;  // per level: existing cells, internal cells
-    if ((r = sc.alloc(&existing, 2 * (uint64_t)L, "xn_build_svo: counters"))) return r;
     uint32_t* nodes = nullptr;
     uint64_t node_bytes = n_total * 40;
     if (!dag && (r = c->device_alloc(reinterpret_cast<void**>(&nodes), node_bytes, "xn_build_svo: node array")))
@@ -962,11 +870,41 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
 
     if (dag) {
         // ---- DAG: classes depth by depth, deepest first
+        // every depth's classes, the hash table of the largest depth, and the
+        // ranks, in one allocation
         std::vector<unsigned long long*> canon(L + 1);
-        for (int d = 0; d <= L; ++d) {
-            uint64_t ids = d < L ? geo[d].n : 8 * geo[L - 1].n;
-            if ((r = sc.alloc(&canon[d], ids, "xn_build_svo: DAG classes"))) return r;
-        }
+        auto table_size = [&](int d) -> uint64_t {
+            const uint64_t count = d < L ? hexist[2 * d] : 8 * hexist[2 * (L - 1) + 1];
+            uint64_t t = 1;
+            while (t < 2 * count) t <<= 1;
+            return count ? t : 0;
+        };
+        Slot* table = nullptr;
+        uint8_t* is_rep = nullptr;
+        unsigned* ins = nullptr;
+        auto plan_dag = [&](unsigned char* base) -> uint64_t {
+            uint64_t used = 0, slots = 1;
+            auto take = [&](uint64_t bytes) -> void* {
+                void* p = base ? base + used : nullptr;
+                used += (bytes + 255) & ~255ull;
+                return p;
+            };
+            for (int d = 0; d <= L; ++d) {
+                canon[d] = static_cast<unsigned long long*>(take((d < L ? geo[d].n : 8 * geo[L - 1].n) * 8));
+                slots = std::max(slots, table_size(d));
+            }
+            // the ranks take the table's place once the classes are known
+            const uint64_t table_at = used;
+            table = static_cast<Slot*>(take(slots * sizeof(Slot)));
+            const uint64_t end = used;
+            used = table_at;
+            is_rep = static_cast<uint8_t*>(take(n_total));
+            ins = static_cast<unsigned*>(take(n_total * 4));
+            return std::max(used, end);
+        };
+        unsigned char* dag_base = nullptr;
+        if ((r = sc.alloc(&dag_base, plan_dag(nullptr), "xn_build_svo: DAG classes"))) return r;
+        plan_dag(dag_base);
         auto level_of = [&](int d) {
             DagLevel a{};
             a.depth = d;
@@ -987,13 +925,8 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
             return a;
         };
         for (int d = L; d >= 0 && e == cudaSuccess; --d) {
-            const uint64_t count = d < L ? hexist[2 * d] : 8 * hexist[2 * (L - 1) + 1];
-            if (count == 0) continue;
-            uint64_t tsize = 1;
-            while (tsize < 2 * count) tsize <<= 1;
-            Slot* table = nullptr;
-            if ((r = c->device_alloc(reinterpret_cast<void**>(&table), tsize * sizeof(Slot), "xn_build_svo: DAG table")))
-                return r;
+            const uint64_t tsize = table_size(d);
+            if (tsize == 0) continue;
             DagLevel a = level_of(d);
             const uint64_t ids = d < L ? geo[d].n : 8 * geo[L - 1].n;
             e = cudaMemsetAsync(table, 0xFF, tsize * sizeof(Slot), s);
@@ -1002,15 +935,8 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
                 dag_lookup_kernel<<<blocks_for(ids, T), T, 0, s>>>(a, table, tsize - 1, counters);
                 e = cudaGetLastError();
             }
-            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
-            c->device_free(table, tsize * sizeof(Slot));
         }
         if (e != cudaSuccess) return cuda_fail(e, "xn_build_svo: DAG classes");
-        uint8_t* is_rep = nullptr;
-        unsigned* ins = nullptr;
-        if ((r = sc.alloc(&is_rep, n_total, "xn_build_svo: DAG ranks")) ||
-            (r = sc.alloc(&ins, n_total, "xn_build_svo: DAG ranks")))
-            return r;
         e = cudaMemsetAsync(is_rep, 0, n_total, s);
         for (int d = L; d >= 0 && e == cudaSuccess; --d) {
             const uint64_t ids = d < L ? geo[d].n : 8 * geo[L - 1].n;
@@ -1646,7 +1572,6 @@ struct StaticLevels {
     unsigned int* counters;
     unsigned long long* leaf_count;
     unsigned long long* existing;
-    unsigned long long* ambig_list;
 };
 
 // The scratch every build needs before the node count is known.
@@ -1665,7 +1590,8 @@ void plan_levels(Arena& a, StaticLevels& p, const LevelGeom* geo, int L, int heu
     p.counters = a.take<unsigned int>(4);
     p.leaf_count = a.take<unsigned long long>(1);
     p.existing = a.take<unsigned long long>(2 * (uint64_t)L);
-    p.ambig_list = heuristic == XN_HEUR_STD_DEV ? a.take<unsigned long long>(big) : nullptr;
+    // part of what std-dev builds are admitted by
+    if (heuristic == XN_HEUR_STD_DEV) a.take<unsigned long long>(big);
 }
 
 int build_static(const uint32_t* d_vox, uint32_t dx, uint32_t dy, uint32_t dz, int type, int heuristic,
@@ -1752,22 +1678,9 @@ int build_static(const uint32_t* d_vox, uint32_t dx, uint32_t dy, uint32_t dz, i
         u.flags = p.flags[d];
         u.chan_diff = (uint32_t)(uint8_t)threshold;
         u.stddev = threshold;
-        u.ambig_count = p.counters;
-        u.ambig_list = p.ambig_list;
-        if (heuristic == XN_HEUR_STD_DEV) {
-            unsigned int amb = 0;
-            e = cudaMemsetAsync(p.counters, 0, 4, s);
-            if (e != cudaSuccess) break;
+        if (heuristic == XN_HEUR_STD_DEV)
             up_level_kernel<XN_HEUR_STD_DEV><<<blocks_for(geo[d].n, T), T, 0, s>>>(u);
-            if ((e = cudaMemcpyAsync(&amb, p.counters, 4, cudaMemcpyDeviceToHost, s)) != cudaSuccess) break;
-            if ((e = cudaStreamSynchronize(s)) != cudaSuccess) break;
-            if (amb) {
-                stddev_fixup_kernel<<<blocks_for(amb, 64), 64, 0, s>>>(u, amb);
-                resize_level_kernel<<<blocks_for(geo[d].n, T), T, 0, s>>>(u);
-            }
-        } else {
-            up_level_kernel<XN_HEUR_CHANNEL_DIFF><<<blocks_for(geo[d].n, T), T, 0, s>>>(u);
-        }
+        else up_level_kernel<XN_HEUR_CHANNEL_DIFF><<<blocks_for(geo[d].n, T), T, 0, s>>>(u);
         e = cudaGetLastError();
     }
     unsigned long long n_total = 0;
