@@ -565,11 +565,11 @@ int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_p
         const float fl = std::sqrt(L.forward[0] * L.forward[0] + L.forward[1] * L.forward[1] +
                                    L.forward[2] * L.forward[2]);
         const float cx = L.translation[0] - 0.5f, cy = L.translation[1] - 0.5f, cz = L.translation[2] - 0.5f;
-        const float width = dmax <= 120u ? std::sqrt(cx * cx + cy * cy + cz * cz) * std::ldexp(1.0f, (int)dmax + 1) /
+        const float width = L.shallow ? std::sqrt(cx * cx + cy * cy + cz * cz) * std::ldexp(1.0f, (int)dmax + 1) /
                                                (fl * (float)L.disp_w)
                                          : 0.0f;
         L.df_packet = pk ? pk[0] != '0' : !(width > 1.0f);
-        L.df_steps = !L.df_packet && L.df_lane_side > 0.0f;
+        L.df_steps = !L.df_packet && L.df_lane_side > 0.0f && L.shallow;
     }
     for (int i = 0; i < 3; ++i) L.dim[i] = v->dim[i];
     return XN_OK;

@@ -378,21 +378,13 @@ constexpr int FIX_BITS = 30;
 constexpr int FIX_DEPTH = 24;
 
 struct LocalPath {
-    static constexpr bool DEEP = true;
     uint32_t n[FIX_DEPTH];
     __device__ __forceinline__ uint32_t& node(int level) { return n[level - 1]; }
 };
 struct SharedPath {
-    static constexpr bool DEEP = true;
     uint32_t* base;  // this thread's column
     uint32_t stride;
     __device__ __forceinline__ uint32_t& node(int level) { return base[(level - 1) * stride]; }
-};
-template <int STRIDE>
-struct ShallowPath {  // octrees of depth <= SHALLOW_ROWS (leaves at most that deep)
-    static constexpr bool DEEP = false;
-    uint32_t* base;  // this thread's column
-    __device__ __forceinline__ uint32_t& node(int level) { return base[(level - 1) * STRIDE]; }
 };
 struct FindPath {
     int depth = -1;          // depth of the last leaf found, -1: none (or too deep to cache)
@@ -417,8 +409,6 @@ __device__ __forceinline__ uint32_t fix_coord(float p) {
 
 __device__ __forceinline__ float fix_to_float(uint32_t v) { return (float)v * (1.0f / 1073741824.0f); }
 
-// Path::DEEP false (octrees of depth <= SHALLOW_ROWS): every node is within
-// the path, so the descent ends at a leaf by itself.
 template <bool COUNT, class Acc, class Path>
 __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Path& pn, V3 pos, V3& base,
                                                 float& side, uint32_t& loads, uint32_t& err) {
@@ -438,7 +428,7 @@ __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Pa
     }
     // the path's levels up to the resumed one are already in place
     for (;; ++level) {
-        if (a.is_leaf(index) || (Path::DEEP && level == FIX_DEPTH)) break;
+        if (a.is_leaf(index) || level == FIX_DEPTH) break;
         const int b = FIX_BITS - 1 - level;
         const uint32_t k = (((px >> b) & 1u) << 2) | (((py >> b) & 1u) << 1) | ((pz >> b) & 1u);
         index = a.child(index, k);
@@ -447,7 +437,7 @@ __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Pa
     const uint32_t keep = ~((1u << (FIX_BITS - level)) - 1u);
     V3 offset = v3(fix_to_float(px & keep), fix_to_float(py & keep), fix_to_float(pz & keep));
     float extent = __uint_as_float((uint32_t)(127 - level) << 23);  // 2^-level
-    if (Path::DEEP && !a.is_leaf(index)) {
+    if (!a.is_leaf(index)) {
         // below depth 24 (deeper than any grid of 2^24 voxels per axis): the
         // reference's float descent
         for (;; ++level) {
@@ -469,7 +459,7 @@ __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Pa
     base = offset;
     side = extent;
     if (COUNT) loads += 2u * (uint32_t)level + 1u;
-    if (!Path::DEEP || level <= FIX_DEPTH) {
+    if (level <= FIX_DEPTH) {
         path.depth = level;
         path.cx = px & keep;
         path.cy = py & keep;
@@ -479,6 +469,54 @@ __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Pa
     }
     return index;
 }
+
+// The same for octrees of depth <= SHALLOW_ROWS, where every node is within the
+// path and 23 bits hold a coordinate: clamp(p, 0, 1) + 1, rounded down, is a
+// float in [1, 2] whose mantissa is floor(p * 2^23) (2 becomes the largest
+// below it), and a cell's origin is the truncated float less 1, exactly.  Both
+// conversions are single additions.  Row 0 of the path is the root.
+template <int STRIDE>
+struct ShallowPath {
+    uint32_t* base;  // this thread's column
+    __device__ __forceinline__ uint32_t& node(int level) { return base[level * STRIDE]; }
+};
+
+__device__ __forceinline__ uint32_t shallow_coord(float p) {
+    return min(__float_as_uint(__fadd_rd(__saturatef(p), 1.0f)), 0x3FFFFFFFu);
+}
+
+template <bool COUNT, class Acc, int STRIDE>
+__device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, ShallowPath<STRIDE>& pn, V3 pos, V3& base,
+                                                float& side, uint32_t& loads, uint32_t&) {
+    const uint32_t px = shallow_coord(pos.x), py = shallow_coord(pos.y), pz = shallow_coord(pos.z);
+    // the leading bits that p shares with the last leaf's origin, at most its depth
+    int level = min(__clz((px ^ path.cx) | (py ^ path.cy) | (pz ^ path.cz)) - 9, path.depth);
+    uint32_t index = pn.node(level);
+    while (!a.is_leaf(index)) {
+        const int b = 22 - level;
+        const uint32_t k = (((px >> b) & 1u) << 2) | (((py >> b) & 1u) << 1) | ((pz >> b) & 1u);
+        index = a.child(index, k);
+        pn.node(++level) = index;
+    }
+    const uint32_t keep = ~0u << (23 - level);
+    path.depth = level;
+    path.cx = px & keep;
+    path.cy = py & keep;
+    path.cz = pz & keep;
+    base = v3(__uint_as_float(path.cx) - 1.0f, __uint_as_float(path.cy) - 1.0f, __uint_as_float(path.cz) - 1.0f);
+    side = __uint_as_float((uint32_t)(127 - level) << 23);  // 2^-level
+    if (COUNT) loads += 2u * (uint32_t)level + 1u;
+    return index;
+}
+
+template <int STRIDE>
+__device__ __forceinline__ void start_path(FindPath& path, ShallowPath<STRIDE>& pn, uint32_t root) {
+    path.depth = 0;
+    path.cx = path.cy = path.cz = 0x3F800000u;
+    pn.node(0) = root;
+}
+template <class Path>
+__device__ __forceinline__ void start_path(FindPath&, Path&, uint32_t) {}
 
 // resources/svo_naive.comp:29-71.  RESUME: each step's find resumes from the
 // previous path (find_cached); else it descends from the root (find), as the
@@ -500,6 +538,7 @@ __device__ V3 trace_naive(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t&
     FindPath path;
     Path local;
     Path& pn = shared_path ? *shared_path : local;
+    start_path(path, pn, a.root());
     while (t < t_max) {
         if (++iter > SVO_MAX_ITER) { err |= 1u; break; }
         V3 p = rd * t + ro;
@@ -779,8 +818,8 @@ __device__ __forceinline__ uint32_t cxor(uint32_t x, bool ax, bool ay, bool az) 
 // tv_max = min(t_max, tc_max) = min(limit, tc_max).  And planes that are 2^-12
 // or more apart have different t's (|t_coeff| 2^-12 is far above the rounding
 // of pos * t_coeff), so tc_max == h only where the child leaves through its
-// parent's exit plane: a parent that was not stacked is never popped, and the
-// stack needs no initial value.
+// parent's exit plane: a parent that the reference does not stack is never
+// popped, so every parent is stacked here, and no row needs an initial value.
 template <bool COUNT, class Acc, class Stacks = LocalStacks>
 __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& err, Stacks* shared_stacks = nullptr) {
     const uint32_t depth = STACK_DEPTH;
@@ -808,7 +847,7 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
     t_max = fminf(t_max, 1.73205078f);  // float(sqrt(3))
 
     uint32_t parent = a.root();
-    uint32_t idx = 0;
+    uint32_t slot = octant_mask;  // the reference's idx ^ octant_mask: the child's index in its parent
     V3 pos = vs(1.0f);
     uint32_t scale = depth - 1;
     float scale_exp2 = 0.5f;
@@ -818,7 +857,7 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
         if (ax) pos.x = 1.5f;
         if (ay) pos.y = 1.5f;
         if (az) pos.z = 1.5f;
-        idx = cxor(idx, ax, ay, az);
+        slot = cxor(slot, ax, ay, az);
     }
     V3 total = vs(0.0f);
     // Between two pops the loop descends at most `depth` times (the scale
@@ -832,14 +871,14 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
         // tv_max <= t_max, the second test alone decides
         float tv_max = fminf(t_max, tc_max);
         if (t_min <= tv_max) {
-            uint32_t child = a.child(parent, idx ^ octant_mask);
+            uint32_t child = a.child(parent, slot);
             if (COUNT) loads += 2;
             if (a.is_leaf(child)) {
                 V3 color = leaf_rgb(a.color(child));
                 if (COUNT) ++loads;
                 total = total + color * (tv_max - t_min);
             } else {
-                if (tc_max < h) {
+                if (!Stacks::T_MAX || tc_max < h) {
                     stk.first(scale) = parent;
                     if constexpr (Stacks::T_MAX) stk.second(scale) = __float_as_uint(t_max);
                 }
@@ -853,7 +892,7 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
                 V3 t_center = v3(__fmaf_rn(t_coeff.x, scale_exp2, t_corner.x), __fmaf_rn(t_coeff.y, scale_exp2, t_corner.y),
                                  __fmaf_rn(t_coeff.z, scale_exp2, t_corner.z));
                 bool ax = t_center.x > t_min, ay = t_center.y > t_min, az = t_center.z > t_min;
-                idx = cxor(0u, ax, ay, az);
+                slot = cxor(octant_mask, ax, ay, az);
                 if (ax) pos.x = pos.x + scale_exp2;
                 if (ay) pos.y = pos.y + scale_exp2;
                 if (az) pos.z = pos.z + scale_exp2;
@@ -868,16 +907,18 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
         if (ay) pos.y = pos.y - scale_exp2;
         if (az) pos.z = pos.z - scale_exp2;
         t_min = tc_max;
-        idx ^= step_mask;
-        if ((idx & step_mask) != 0) {
+        slot ^= step_mask;
+        if (((slot ^ octant_mask) & step_mask) != 0) {
             // POP
             if (++pops > SVO_MAX_ITER) { err |= 1u; break; }
             uint32_t xx = __float_as_uint(pos.x) ^ __float_as_uint(pos.x + scale_exp2);
             uint32_t xy = __float_as_uint(pos.y) ^ __float_as_uint(pos.y + scale_exp2);
             uint32_t xz = __float_as_uint(pos.z) ^ __float_as_uint(pos.z + scale_exp2);
             uint32_t dbits = (ax ? xx : 0u) | (ay ? xy : 0u) | (az ? xz : 0u);
-            scale = (__float_as_uint(__uint2float_rn(dbits)) >> 23) - 127u;
-            if (scale >= depth) break;  // the loop condition ends the ray
+            // the highest bit that changed; beyond the mantissa, the loop
+            // condition ends the ray (dbits < 2^23 as a float is exact)
+            if (dbits - 1u >= (1u << STACK_DEPTH) - 1u) break;
+            scale = (__float_as_uint(__uint_as_float(dbits | 0x4B000000u) - 8388608.0f) >> 23) - 127u;
             scale_exp2 = __uint_as_float((scale - depth + 127u) << 23);
             parent = stk.first(scale);
             if constexpr (Stacks::T_MAX) t_max = __uint_as_float(stk.second(scale));
@@ -885,7 +926,7 @@ __device__ V3 trace_esvo(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32_t& 
             uint32_t shy = __float_as_uint(pos.y) >> scale;
             uint32_t shz = __float_as_uint(pos.z) >> scale;
             pos = v3(__uint_as_float(shx << scale), __uint_as_float(shy << scale), __uint_as_float(shz << scale));
-            idx = (shx & 1u) * 4u + (shy & 1u) * 2u + (shz & 1u);
+            slot = ((shx & 1u) * 4u + (shy & 1u) * 2u + (shz & 1u)) ^ octant_mask;
             h = 0.0f;
         }
     }
@@ -902,15 +943,24 @@ __device__ __forceinline__ uint32_t find_relative(const Acc& a, uint32_t parent,
     // by 2^d (both built from their exponents), as in gl_mod_pow2
     float extent, inv = 0.0f;
     bool ex = false;
-    if (d <= 124u) {
+    if (d <= (uint32_t)SHALLOW_ROWS) {
+        // offset and 1.5 * 2^(23-d) have a sum whose last place is 2^-d, so
+        // rounding it down snaps the offset down to a multiple of 2^-d
+        // (offsets are within the octree or one cell beside it)
         extent = __uint_as_float((127u - d) << 23);
-        inv = __uint_as_float((127u + d) << 23);
-        ex = true;
+        const float c = __uint_as_float(((150u - d) << 23) | 0x400000u);
+        offset = v3(__fadd_rd(offset.x, c) - c, __fadd_rd(offset.y, c) - c, __fadd_rd(offset.z, c) - c);
     } else {
-        extent = ldexpf(1.0f, -(int)(d > 1000u ? 1000u : d));
+        if (d <= 124u) {
+            extent = __uint_as_float((127u - d) << 23);
+            inv = __uint_as_float((127u + d) << 23);
+            ex = true;
+        } else {
+            extent = ldexpf(1.0f, -(int)(d > 1000u ? 1000u : d));
+        }
+        offset = v3(snap_down_pow2(offset.x, extent, inv, ex), snap_down_pow2(offset.y, extent, inv, ex),
+                    snap_down_pow2(offset.z, extent, inv, ex));
     }
-    offset = v3(snap_down_pow2(offset.x, extent, inv, ex), snap_down_pow2(offset.y, extent, inv, ex),
-                snap_down_pow2(offset.z, extent, inv, ex));
     for (int level = 0;; ++level) {
         if (COUNT) ++loads;
         if (a.is_leaf(parent)) {
@@ -1143,7 +1193,7 @@ __device__ __forceinline__ void svo_pixel(const Frame& f, const Acc& a, const Ou
         SharedPath sp{s_path + threadIdx.x, BLOCK_THREADS};
         total = trace_naive<COUNT, Acc, true, SharedPath>(a, f.translation, rd, loads, err, &sp);
     } else if constexpr (TRAV == XN_TRAV_SVO_NAIVE_SHALLOW) {
-        __shared__ uint32_t s_path[SHALLOW_ROWS * BLOCK_THREADS];
+        __shared__ uint32_t s_path[(SHALLOW_ROWS + 1) * BLOCK_THREADS];
         ShallowPath<BLOCK_THREADS> sp{s_path + threadIdx.x};
         total = trace_naive<COUNT, Acc, true, ShallowPath<BLOCK_THREADS>>(a, f.translation, rd, loads, err, &sp);
     } else if (TRAV == XN_TRAV_SVO_NAIVE_ROOT) {
@@ -1379,11 +1429,12 @@ __device__ V3 trace_df_steps(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32
             const uint32_t st = stk.second(sp);
             todo = st & 0xFFu;
             depth = st >> 8;
-            // 2^-depth and 2^depth from their exponents (depths are at most
-            // 120 here); the snap down is the reference's pos - mod(pos, 2 side)
-            const float s2 = __uint_as_float((127u - depth) << 23), inv = __uint_as_float((127u + depth) << 23);
-            side = s2 * 0.5f;
-            origin = v3(s2 * floorf(origin.x * inv), s2 * floorf(origin.y * inv), s2 * floorf(origin.z * inv));
+            // 2^-(depth + 1) from its exponent; the reference's pos - mod(pos,
+            // 2 side) is the origin rounded down to a multiple of 2^-depth
+            // (depths are at most SHALLOW_ROWS: see find_relative)
+            side = __uint_as_float((126u - depth) << 23);
+            const float c = __uint_as_float(((150u - depth) << 23) | 0x400000u);
+            origin = v3(__fadd_rd(origin.x, c) - c, __fadd_rd(origin.y, c) - c, __fadd_rd(origin.z, c) - c);
         }
     }
     return total;
@@ -1567,20 +1618,25 @@ __global__ void __launch_bounds__(SHARED_BLOCK) shared_stack_kernel(Frame f, Acc
     write_outputs(f, o, ix, iy, total * voxel_emission_coeff(f, rd), loads, err);
 }
 
+// Blocks of 128: with 7 KB of stacks a block, smaller blocks no longer cost L1
+// (esvo, Mrays/s, 512x361x512 CT shell at 1920x1080 and 512^3 gas field: blocks
+// of 256 1996 and 570, of 128 2100 and 580, of 64 2048 and 569).  Asking for
+// eight resident blocks instead of leaving it open (40 registers) is 1-3 %
+// better on small frames.
 template <bool COUNT>
-__global__ void __launch_bounds__(SHARED_BLOCK) esvo_shallow_kernel(Frame f, CompactNodes a, Outputs o) {
-    __shared__ uint32_t s_a[SHALLOW_ROWS * SHARED_BLOCK];
+__global__ void __launch_bounds__(BLOCK_THREADS, 8) esvo_shallow_kernel(Frame f, CompactNodes a, Outputs o) {
+    __shared__ uint32_t s_a[SHALLOW_ROWS * BLOCK_THREADS];
     fill_unorm_lut();
     uint32_t ix, iy;
-    if (!pixel_of_thread_bt<SHARED_BLOCK>(f, ix, iy)) return;
-    NodeStack<SHARED_BLOCK> stk{s_a + threadIdx.x};
+    if (!pixel_of_thread(f, ix, iy)) return;
+    NodeStack<BLOCK_THREADS> stk{s_a + threadIdx.x};
     const V3 rd = primary_ray(f, ix, iy);
     uint32_t loads = 0, err = 0;
     // resources/esvo.comp:148-152
     V3 ro = f.translation + vs(1.0f);
     const float t0 = aabb_entry(vs(1.0f), vs(2.0f), ro, rd);
     ro = ro + rd * fmaxf(t0, 0.0f);
-    const V3 total = trace_esvo<COUNT, CompactNodes, NodeStack<SHARED_BLOCK>>(a, ro, rd, loads, err, &stk);
+    const V3 total = trace_esvo<COUNT, CompactNodes, NodeStack<BLOCK_THREADS>>(a, ro, rd, loads, err, &stk);
     write_outputs(f, o, ix, iy, total * voxel_emission_coeff(f, rd), loads, err);
 }
 
@@ -1682,8 +1738,8 @@ cudaError_t launch_render(const RenderLaunch& L, cudaStream_t stream) {
             else shared_stack_kernel<XN_TRAV_ESVO, false><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
         } else {
             const CompactNodes acc{L.inner, L.inner_depth};
-            if (L.shallow && count) esvo_shallow_kernel<true><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
-            else if (L.shallow) esvo_shallow_kernel<false><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
+            if (L.shallow && count) esvo_shallow_kernel<true><<<grid, BLOCK_THREADS, 0, stream>>>(f, acc, o);
+            else if (L.shallow) esvo_shallow_kernel<false><<<grid, BLOCK_THREADS, 0, stream>>>(f, acc, o);
             else if (count) shared_stack_kernel<XN_TRAV_ESVO, true><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
             else shared_stack_kernel<XN_TRAV_ESVO, false><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
         }
