@@ -118,6 +118,7 @@ XN_API int xn_create(int device, uint64_t hbm_budget_bytes, xn_ctx** out) {
         xn_destroy(reinterpret_cast<xn_ctx*>(c));
         return r;
     }
+    c->sm_count();  // known before any launch, whichever thread makes it
     r = c->device_alloc(reinterpret_cast<void**>(&c->d_err), sizeof(uint32_t), "xn_create: error word");
     if (r) { xn_destroy(reinterpret_cast<xn_ctx*>(c)); return r; }
     cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream);
@@ -483,6 +484,26 @@ XN_API int xn_volume_info_get(const xn_volume* h, xn_volume_info* info) {
 
 namespace xn {
 
+// Frames too small to fill the GPU with warps of 32 rays are traced by warps of
+// 16, 8, 4 or 2 (1 to 4; 0: 32).  Their time is the longest warp's, and a warp
+// runs every path that any of its rays takes at a step, so fewer rays a warp
+// are fewer instructions; with more warps the idle lanes cost more than that
+// gives, the sooner the more of the frame the volume covers (`zoom`: the
+// volume's width over the frame's) and the more alike the rays are.  Warps an SM
+// up to which every traversal gained, measured on 96x96 to 340x340 frames of
+// 48^3 to 512^3 blobs, gas fields and CT shells: from inside 8 (96x96 with warps
+// of 8: 1.0-1.5x), filling the frame 16 (139x139 with warps of 8: 1.02-1.2x), or
+// 27 where the volume is large and rays long (181x181 with warps of 8: svo-naive
+// and svo-rope 1.45-1.7x, the others 1.1-1.2x), from farther away 24 (160x120
+// with warps of 8: 1.1-1.3x) and 48 (139x139 with warps of 4: 1.4-2.5x; 256x256
+// of 16: 1.06-1.3x).  At twice these counts some lose 10-40 %.
+static uint32_t narrow_warps(uint64_t rays, int sms, bool large, float zoom) {
+    const uint32_t limit = zoom < 0.77f ? (large ? 48 : 24) : zoom < 1.15f ? (large ? 27 : 16) : 8;
+    for (uint32_t n = 4; n > 0; --n)
+        if (rays <= (uint64_t)sms * limit * (32u >> n)) return n;
+    return 0;
+}
+
 int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_params* p, RenderLaunch& L) {
     if (traversal < XN_DDA || traversal > XN_SVO_ROPE) return fail(XN_ERR_ARG, "invalid traversal %d", traversal);
     if (traversal == XN_DDA && v->kind != XN_VOLUME_GRID)
@@ -515,6 +536,21 @@ int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_p
     L.disp_y = p->display_region.y;
     L.disp_w = p->display_region.width;
     L.disp_h = p->display_region.height;
+    {
+        // an octree spans [0, 1] (and its side is the power of two above its
+        // grid's); a grid spans its sides over the longest
+        const bool grid = v->kind == XN_VOLUME_GRID;
+        const uint32_t side = v->dim[0] > v->dim[1] ? (v->dim[0] > v->dim[2] ? v->dim[0] : v->dim[2])
+                                                    : (v->dim[1] > v->dim[2] ? v->dim[1] : v->dim[2]);
+        float d2 = 0.0f, f2 = 0.0f;
+        for (int i = 0; i < 3; ++i) {
+            const float c = L.translation[i] - (grid ? 0.5f * (float)v->dim[i] / (float)side : 0.5f);
+            d2 += c * c;
+            f2 += L.forward[i] * L.forward[i];
+        }
+        L.narrow = narrow_warps((uint64_t)L.out_w * L.out_h, v->ctx->sm_count(), side >= (grid ? 128u : 256u),
+                                std::sqrt(f2 / d2));
+    }
     if (v->kind == XN_VOLUME_GRID) {
         L.grid = v->data;
         L.tex = v->tex;
@@ -569,6 +605,7 @@ int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_p
                                                (fl * (float)L.disp_w)
                                          : 0.0f;
         L.df_packet = pk ? pk[0] != '0' : !(width > 1.0f);
+        L.df_narrow = !pk && L.df_lane_side > 0.0f && L.shallow;
         L.df_steps = !L.df_packet && L.df_lane_side > 0.0f && L.shallow;
     }
     for (int i = 0; i < 3; ++i) L.dim[i] = v->dim[i];

@@ -1074,11 +1074,17 @@ __device__ __forceinline__ bool pixel_of_thread_bt(const Frame& f, uint32_t& ix,
     return ix < f.out_w && iy < f.out_h;
 }
 
+// Narrow warps (f.narrow): 8x4, 4x4, 4x2, 2x2 or 2x1 pixels traced by a warp's
+// first lanes.
+__host__ __device__ __forceinline__ uint32_t warp_tile_w(uint32_t narrow) { return 8u >> ((narrow + 1u) >> 1); }
+__host__ __device__ __forceinline__ uint32_t warp_tile_h(uint32_t narrow) { return 4u >> (narrow >> 1); }
+
 __device__ __forceinline__ bool pixel_of_thread(const Frame& f, uint32_t& ix, uint32_t& iy) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    ix = blockIdx.x * TILE_W + (warp & 1u) * 8u + (lane & 7u);
-    iy = blockIdx.y * TILE_H + (warp >> 1) * 4u + (lane >> 3);
-    return ix < f.out_w && iy < f.out_h;
+    const uint32_t tw = warp_tile_w(f.narrow), th = warp_tile_h(f.narrow);
+    ix = (blockIdx.x * 2u + (warp & 1u)) * tw + (lane & (tw - 1u));
+    iy = (blockIdx.y * 2u + (warp >> 1)) * th + (lane >> (3u - ((f.narrow + 1u) >> 1)));
+    return lane < tw * th && ix < f.out_w && iy < f.out_h;
 }
 
 __device__ __forceinline__ void write_outputs(const Frame& f, const Outputs& o, uint32_t ix, uint32_t iy, V3 color,
@@ -1125,7 +1131,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS) dda_tex_kernel(Frame f, cudaTex
                                                                uint32_t dy, uint32_t dz, Outputs o) {
     if (NORM == TEX_RAW) fill_unorm_lut();
     uint32_t ix, iy;
-    if (!pixel_of_thread_ww<WW>(f, ix, iy)) return;
+    if (!(WW == 8 ? pixel_of_thread(f, ix, iy) : pixel_of_thread_ww<WW>(f, ix, iy))) return;
     uint32_t m = max(dx, max(dy, dz));
     float side = (float)m;
     V3 ro = f.translation * side;
@@ -1682,7 +1688,12 @@ cudaError_t launch_render(const RenderLaunch& L, cudaStream_t stream) {
     f.disp_w = L.disp_w;
     f.disp_h = L.disp_h;
     Outputs o{static_cast<uint32_t*>(L.d_rgba), L.d_emission, L.d_loads, L.d_err_word};
-    dim3 grid((L.out_w + TILE_W - 1) / TILE_W, (L.out_h + TILE_H - 1) / TILE_H);
+    // the warp walk needs whole warps; on the smallest frames one ray per lane
+    // in narrow warps is the quicker svo-df at any pixel width
+    const bool packet = L.df_packet && !(L.df_narrow && L.narrow == 4);
+    f.narrow = L.traversal == XN_TRAV_SVO_DF && packet && L.layout == XN_LAYOUT_COMPACT && L.depth_consistent ? 0 : L.narrow;
+    const uint32_t bw = 2 * warp_tile_w(f.narrow), bh = 2 * warp_tile_h(f.narrow);
+    dim3 grid((L.out_w + bw - 1) / bw, (L.out_h + bh - 1) / bh);
     const bool count = L.d_loads != nullptr;
     if (L.traversal == XN_TRAV_DDA && L.tex) {
         const cudaTextureObject_t t = L.tex;
@@ -1743,12 +1754,12 @@ cudaError_t launch_render(const RenderLaunch& L, cudaStream_t stream) {
             else if (count) shared_stack_kernel<XN_TRAV_ESVO, true><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
             else shared_stack_kernel<XN_TRAV_ESVO, false><<<grid16, SHARED_BLOCK, 0, stream>>>(f, acc, o);
         }
-    } else if (L.traversal == XN_TRAV_SVO_DF && L.df_steps && !L.shared_stacks && L.layout == XN_LAYOUT_COMPACT &&
+    } else if (L.traversal == XN_TRAV_SVO_DF && (L.df_steps || (L.df_packet && !packet)) && !L.shared_stacks && L.layout == XN_LAYOUT_COMPACT &&
                L.depth_consistent) {
         const CompactNodes acc{L.inner, L.inner_depth};
         if (count) df_steps_kernel<true><<<grid, BLOCK_THREADS, 0, stream>>>(f, acc, o);
         else df_steps_kernel<false><<<grid, BLOCK_THREADS, 0, stream>>>(f, acc, o);
-    } else if (L.traversal == XN_TRAV_SVO_DF && L.df_packet && L.layout == XN_LAYOUT_COMPACT && L.depth_consistent) {
+    } else if (L.traversal == XN_TRAV_SVO_DF && packet && L.layout == XN_LAYOUT_COMPACT && L.depth_consistent) {
         const CompactNodes acc{L.inner, L.inner_depth};
         if (L.df_lane_levels == 2) {
             if (count) df_packet_kernel<true, CompactNodes, 2><<<grid, BLOCK_THREADS, 0, stream>>>(f, acc, o, L.df_lane_side);
@@ -1856,6 +1867,7 @@ __device__ __forceinline__ Frame frame_of(const BatchJob& J) {
     f.disp_y = J.disp_y;
     f.disp_w = J.disp_w;
     f.disp_h = J.disp_h;
+    f.narrow = 0;
     return f;
 }
 

@@ -56,6 +56,8 @@ struct RenderLaunch {
     int shallow;                  // depth consistent, and no leaf deeper than XN_SHALLOW_DEPTH
     int naive_resume;             // svo-naive's find resumes from the previous step's path
     int df_packet;                // masked svo-df walked by the whole warp (df_packet_kernel)
+    int df_narrow;                // the choice between the two forms of svo-df is free: narrow frames take df_steps
+    uint32_t narrow;              // warps of 32 >> narrow rays (xn_device.cuh Frame)
     int df_steps;                 // masked svo-df one ray per lane, every step alike (df_steps_kernel)
     float df_lane_side;           // child size of the nodes below which the lanes walk alone: 2^-D
                                   // (one level; D the deepest internal node's depth) or 2^-(D-1)
