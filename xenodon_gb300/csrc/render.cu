@@ -475,10 +475,11 @@ __device__ __forceinline__ uint32_t find_cached(const Acc& a, FindPath& path, Pa
 // float in [1, 2] whose mantissa is floor(p * 2^23) (2 becomes the largest
 // below it), and a cell's origin is the truncated float less 1, exactly.  Both
 // conversions are single additions.  Row 0 of the path is the root.
-template <int STRIDE>
+template <int STRIDE>  // between a thread's rows; 0: `stride`
 struct ShallowPath {
     uint32_t* base;  // this thread's column
-    __device__ __forceinline__ uint32_t& node(int level) { return base[level * STRIDE]; }
+    uint32_t stride = STRIDE;
+    __device__ __forceinline__ uint32_t& node(int level) { return base[level * (STRIDE ? STRIDE : stride)]; }
 };
 
 __device__ __forceinline__ uint32_t shallow_coord(float p) {
@@ -652,11 +653,14 @@ struct SharedStacks {
 // esvo's parents alone, for octrees whose internal nodes are at most
 // SHALLOW_ROWS - 1 deep: scales STACK_DEPTH - 1 down to STACK_DEPTH -
 // SHALLOW_ROWS, one column of shared memory per thread.
-template <int STRIDE>
+template <int STRIDE>  // between a thread's rows; 0: `stride`
 struct NodeStack {
     static constexpr bool T_MAX = false;
     uint32_t* a;  // this thread's column
-    __device__ __forceinline__ uint32_t& first(uint32_t i) { return a[(i - (STACK_DEPTH - SHALLOW_ROWS)) * STRIDE]; }
+    uint32_t stride = STRIDE;
+    __device__ __forceinline__ uint32_t& first(uint32_t i) {
+        return a[(i - (STACK_DEPTH - SHALLOW_ROWS)) * (STRIDE ? STRIDE : stride)];
+    }
     __device__ __forceinline__ uint32_t& second(uint32_t i) { return first(i); }
 };
 
@@ -1419,7 +1423,7 @@ __device__ V3 trace_df_steps(const Acc& a, V3 ro, V3 rd, uint32_t& loads, uint32
             // node (the reference pushes it unless k == 7)
             if (COUNT) loads += 8u + (k != 7u ? 1u : 0u);
             if (mask) {
-                if (sp >= STACK_DEPTH) { err |= 2u; break; }
+                // (at most SHALLOW_ROWS - 1 nodes are on the path)
                 stk.first(sp) = node;
                 stk.second(sp) = mask | (depth << 8);
                 ++sp;
@@ -1582,8 +1586,8 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 5) df_packet_kernel(Frame f, Ac
 
 template <bool COUNT, class Acc>
 __global__ void __launch_bounds__(BLOCK_THREADS) df_steps_kernel(Frame f, Acc a, Outputs o) {
-    __shared__ uint32_t s_a[STACK_DEPTH * BLOCK_THREADS];
-    __shared__ uint32_t s_b[STACK_DEPTH * BLOCK_THREADS];
+    __shared__ uint32_t s_a[SHALLOW_ROWS * BLOCK_THREADS];
+    __shared__ uint32_t s_b[SHALLOW_ROWS * BLOCK_THREADS];
     fill_unorm_lut();
     uint32_t ix, iy;
     if (!pixel_of_thread(f, ix, iy)) return;
@@ -1833,6 +1837,7 @@ BatchJob make_batch_job(const RenderLaunch& L) {
     // the batch's svo-df form walks one level per lane (its blocks of up to
     // 1024 threads leave 64 registers a thread): child size 2^-D
     j.df_steps = L.df_steps;
+    j.shallow = L.shallow;
     j.df_lane_side = L.df_lane_levels == 2 ? L.df_lane_side * 0.5f : L.df_lane_side;
     return j;
 }
@@ -1997,6 +2002,19 @@ __device__ __forceinline__ uint32_t render_job_pixel_spec(const BatchJob& J, uin
                 color = trace_dda_tex<false, TEX_PACKED>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err) * ec;
             else
                 color = trace_dda_tex<false, TEX_RAW>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err) * ec;
+        } else if constexpr (SPEC == XN_BATCH_ESVO_SHALLOW) {
+            NodeStack<0> nodes{stk->a, stk->stride};
+            V3 ro = f.translation + vs(1.0f);
+            const float t0 = aabb_entry(vs(1.0f), vs(2.0f), ro, rd);
+            ro = ro + rd * fmaxf(t0, 0.0f);
+            color = trace_esvo<false, CompactNodes, NodeStack<0>>(CompactNodes{J.inner, J.inner_depth}, ro, rd, loads,
+                                                                  err, &nodes) *
+                    voxel_emission_coeff(f, rd);
+        } else if constexpr (SPEC == XN_BATCH_NAIVE_SHALLOW) {
+            ShallowPath<0> path{stk->a, stk->stride};
+            color = trace_naive<false, CompactNodes, true, ShallowPath<0>>(CompactNodes{J.inner, J.inner_depth},
+                                                                           f.translation, rd, loads, err, &path) *
+                    voxel_emission_coeff(f, rd);
         } else if constexpr (SPEC == XN_BATCH_DF_STEPS) {
             color = trace_df_steps<false>(CompactNodes{J.inner, J.inner_depth}, f.translation, rd, loads, err, *stk) *
                     voxel_emission_coeff(f, rd);
@@ -2021,15 +2039,27 @@ constexpr int batch_min_blocks(int spec) {
     return spec == XN_BATCH_DDA_TEX_NORM || spec == XN_BATCH_DDA_TEX_RAW ? 2 : 1;
 }
 
+// Rows of dynamic shared memory per thread: one column of stack or path, or two
+// of batch_rows / 2 each.
+__host__ __device__ constexpr int batch_rows(int spec) {
+    switch (spec) {
+    case XN_BATCH_ESVO_SHALLOW: return SHALLOW_ROWS;
+    case XN_BATCH_NAIVE_SHALLOW: return SHALLOW_ROWS + 1;
+    case XN_BATCH_DF_STEPS: return 2 * SHALLOW_ROWS;
+    case XN_BATCH_ANY:
+    case XN_BATCH_ESVO:
+    case XN_BATCH_DF: return 2 * STACK_DEPTH;
+    default: return 0;
+    }
+}
+
 template <int TW, int SPEC>
 __global__ void __launch_bounds__(1024, batch_min_blocks(SPEC)) batch_kernel(const BatchHeader* hdr, const BatchJob* jobs,
                                                      unsigned long long* queue, uint32_t chunk, uint32_t* err_word) {
     fill_unorm_lut();
     constexpr int TH = 32 / TW;
-    // esvo and svo-df stacks: two columns per thread in dynamic shared memory
-    // (2 * STACK_DEPTH words a thread, given at launch for the forms that use them)
     extern __shared__ uint32_t batch_stacks[];
-    SharedStacks stk{batch_stacks + threadIdx.x, batch_stacks + STACK_DEPTH * blockDim.x + threadIdx.x, blockDim.x};
+    SharedStacks stk{batch_stacks + threadIdx.x, batch_stacks + batch_rows(SPEC) / 2 * blockDim.x + threadIdx.x, blockDim.x};
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned long long total = hdr->total_tiles;
     const uint32_t n = hdr->n_jobs;
@@ -2069,7 +2099,7 @@ __global__ void __launch_bounds__(1024, batch_min_blocks(SPEC)) batch_grid_kerne
     fill_unorm_lut();
     constexpr int TH = 32 / TW;
     extern __shared__ uint32_t batch_stacks[];
-    SharedStacks stk{batch_stacks + threadIdx.x, batch_stacks + STACK_DEPTH * blockDim.x + threadIdx.x, blockDim.x};
+    SharedStacks stk{batch_stacks + threadIdx.x, batch_stacks + batch_rows(SPEC) / 2 * blockDim.x + threadIdx.x, blockDim.x};
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned long long t =
         (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -2092,19 +2122,15 @@ __global__ void __launch_bounds__(1024, batch_min_blocks(SPEC)) batch_grid_kerne
     if (err) atomicOr(err_word, err);
 }
 
-constexpr bool batch_needs_stacks(int spec) {
-    return spec == XN_BATCH_ANY || spec == XN_BATCH_ESVO || spec == XN_BATCH_DF || spec == XN_BATCH_DF_STEPS;
-}
-
 template <int TW, int SPEC>
 static cudaError_t launch_batch_tws(const void* table, unsigned long long* q, uint32_t* err, uint32_t threads,
                                     uint32_t blocks, uint32_t chunk, cudaStream_t s) {
     const BatchHeader* hdr = static_cast<const BatchHeader*>(table);
     const BatchJob* jobs = reinterpret_cast<const BatchJob*>(hdr + 1);
-    const size_t smem = batch_needs_stacks(SPEC) ? (size_t)2 * STACK_DEPTH * 4 * threads : 0;
+    const size_t smem = (size_t)batch_rows(SPEC) * 4 * threads;
     if (chunk == 0) {
         // queue-less form: one warp per tile; `blocks` is the grid for all tiles
-        if (smem > 48 * 1024) {
+        if (smem > 40 * 1024) {  // with the static part, past the default limit
             const cudaError_t e =
                 cudaFuncSetAttribute(batch_grid_kernel<TW, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
             if (e != cudaSuccess) return e;
@@ -2112,7 +2138,7 @@ static cudaError_t launch_batch_tws(const void* table, unsigned long long* q, ui
         batch_grid_kernel<TW, SPEC><<<blocks, threads, smem, s>>>(hdr, jobs, err);
         return cudaGetLastError();
     }
-    if (smem > 48 * 1024) {
+    if (smem > 40 * 1024) {  // with the static part, past the default limit
         const cudaError_t e =
             cudaFuncSetAttribute(batch_kernel<TW, SPEC>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return e;
@@ -2131,6 +2157,10 @@ static cudaError_t launch_batch_tw(const void* table, unsigned long long* q, uin
     case XN_BATCH_NAIVE: return launch_batch_tws<TW, XN_BATCH_NAIVE>(table, q, err, threads, blocks, chunk, s);
     case XN_BATCH_DF: return launch_batch_tws<TW, XN_BATCH_DF>(table, q, err, threads, blocks, chunk, s);
     case XN_BATCH_DF_STEPS: return launch_batch_tws<TW, XN_BATCH_DF_STEPS>(table, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_ESVO_SHALLOW:
+        return launch_batch_tws<TW, XN_BATCH_ESVO_SHALLOW>(table, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_NAIVE_SHALLOW:
+        return launch_batch_tws<TW, XN_BATCH_NAIVE_SHALLOW>(table, q, err, threads, blocks, chunk, s);
     case XN_BATCH_ROPE: return launch_batch_tws<TW, XN_BATCH_ROPE>(table, q, err, threads, blocks, chunk, s);
     default: return launch_batch_tws<TW, XN_BATCH_ANY>(table, q, err, threads, blocks, chunk, s);
     }

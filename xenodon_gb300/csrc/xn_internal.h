@@ -94,6 +94,7 @@ struct alignas(16) BatchJob {
     int32_t depth_consistent;
     int32_t form;  // XN_BATCH_* form of this job (batch_spec)
     int32_t df_steps;    // svo-df: one ray per lane (trace_df_steps)
+    int32_t shallow;     // octree of depth <= XN_SHALLOW_DEPTH
     float df_lane_side;  // svo-df: child size 2^-D of the nodes whose children the lanes walk alone, or 0
     unsigned long long tex;
     const void* grid;
@@ -116,7 +117,9 @@ BatchJob make_batch_job(const RenderLaunch& L);
 // Batch kernel forms: one traversal (and layout) inlined when every job of
 // the batch shares it, else the generic per-pixel dispatch.
 enum { XN_BATCH_ANY = 0, XN_BATCH_DDA_TEX_NORM, XN_BATCH_DDA_TEX_RAW, XN_BATCH_ESVO, XN_BATCH_NAIVE, XN_BATCH_DF,
-       XN_BATCH_ROPE, XN_BATCH_DF_STEPS, XN_BATCH_FORMS };
+       XN_BATCH_ROPE, XN_BATCH_DF_STEPS, XN_BATCH_FORMS,
+       // launches, not forms of a job: every job of XN_BATCH_ESVO / XN_BATCH_NAIVE is on a shallow octree
+       XN_BATCH_ESVO_SHALLOW = XN_BATCH_FORMS, XN_BATCH_NAIVE_SHALLOW };
 // The form a job needs (XN_BATCH_*).
 int batch_spec(const BatchJob& j);
 // Launches the persistent kernel over a job table already in device memory
