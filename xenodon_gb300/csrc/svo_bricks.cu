@@ -46,13 +46,13 @@ constexpr uint32_t LEAF = 0x80000000u;
 constexpr unsigned long long NONE = ~0ull;
 constexpr uint32_t FULL = 0xFFFFFFFFu;
 constexpr uint8_t F_LEAF = 1, F_INSIDE = 2;
-constexpr int BT = 128;          // a block: 4 warps, each two octants (8^3 voxels) of the brick that are neighbours in x
+constexpr int BT = 128;          // a scan block: 4 warps, each two octants (8^3 voxels) of the brick that are neighbours in x
 constexpr uint32_t ROOT_BIT = 256;
-constexpr uint64_t TOP_CELLS = 4096;
+constexpr uint64_t TOP_CELLS = 1024;
 
 // Octants o, groups g (4^3 voxels, eight an octant) and cells m (2^3 voxels,
 // 64 an octant, m = 8 g + child) are in child order: x is the high digit.
-struct BrickRec {
+struct alignas(16) BrickRec {
     unsigned long long l1[8];  // per octant: internal cells of 2^3 voxels
     unsigned long long l2;     // byte o: internal groups of octant o
     uint16_t pre[8];           // internal nodes of the brick before octant o in post-order
@@ -182,12 +182,12 @@ __device__ __forceinline__ Part part_shfl(const Part& p, int mask) {
 
 // construct()'s decision (OctreeConstruction.h:141-171) for a cell inside a
 // brick: internal unless it is a leaf or outside the grid.  Cells of a brick
-// that lies inside the grid as a whole (`whole`) skip the geometry.
-template <int HEUR>
-__device__ __forceinline__ bool cell_internal(const Levels& a, bool whole, uint32_t x, uint32_t y, uint32_t z,
+// that lies inside the grid as a whole (WHOLE) skip the geometry.
+template <int HEUR, bool WHOLE>
+__device__ __forceinline__ bool cell_internal(const Levels& a, uint32_t x, uint32_t y, uint32_t z,
                                               uint32_t e, const Part& p, uint32_t s0, uint32_t s1, uint32_t s2,
                                               uint32_t s3) {
-    if (!whole) {
+    if (!WHOLE) {
         if (x >= a.g.dx || y >= a.g.dy || z >= a.g.dz) return false;
         if (x + e > a.g.dx || y + e > a.g.dy || z + e > a.g.dz) return true;  // partly inside: always split
     }
@@ -299,6 +299,86 @@ struct OctantSums {
     uint32_t q;
 };
 
+// One octant of a brick by one warp: the lane's 16 voxels are q, h is the
+// octant's place in x.
+template <int HEUR, bool WHOLE>
+__device__ __forceinline__ void scan_octant(const Levels& a, const uint4 q[4], const Place& pl, uint32_t lane, uint32_t OX,
+                                            uint32_t OY, uint32_t OZ, OctantSums& os, unsigned long long& l1,
+                                            uint32_t& l2, uint32_t& l3) {
+    if (WHOLE) {
+        // an octant of one value, as most of a sparse volume is: a leaf
+        uint32_t dif = (q[0].y ^ q[0].x) | (q[0].z ^ q[0].x) | (q[0].w ^ q[0].x);
+#pragma unroll
+        for (int r = 1; r < 4; ++r)
+            dif |= (q[r].x ^ q[0].x) | (q[r].y ^ q[0].x) | (q[r].z ^ q[0].x) | (q[r].w ^ q[0].x);
+        dif |= __shfl_sync(FULL, q[0].x, 0) ^ q[0].x;
+        if (!__any_sync(FULL, dif != 0)) {
+            if (lane == 0) {
+                const uint32_t v = q[0].x;
+#pragma unroll
+                for (int c = 0; c < 4; ++c) os.s[c] = 512u * ((v >> (8 * c)) & 0xFFu);
+                os.mn = os.mx = v;
+                os.q = 512u * __dp4a(v, v, 0u);
+                l1 = 0;
+                l2 = l3 = 0;
+            }
+            return;
+        }
+    }
+    const uint32_t x = OX + pl.cx * 2, y = OY + pl.cy * 2, z = OZ + pl.cz * 2;
+    Part group = part_empty<HEUR>();
+    uint32_t in[2];
+#pragma unroll
+    for (uint32_t c = 0; c < 2; ++c) {
+        Part p = part_empty<HEUR>();
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            const bool valid = WHOLE || (x + 2 * c + (k >> 2) < a.g.dx && y + ((k >> 1) & 1u) < a.g.dy &&
+                                         z + (k & 1u) < a.g.dz);
+            part_add<HEUR>(p, cell_voxel(q, c, k), valid);
+        }
+        const bool internal = cell_internal<HEUR, WHOLE>(a, x + 2 * c, y, z, 2, p, p.s02 & 0xFFFFu, p.s13 & 0xFFFFu,
+                                                         p.s02 >> 16, p.s13 >> 16);
+        in[c] = __ballot_sync(FULL, internal);
+        if (c == 0) group = p;
+        else part_merge<HEUR>(group, p);
+    }
+    // groups: the four lanes of one
+    part_merge<HEUR>(group, part_shfl<HEUR>(group, 1));
+    part_merge<HEUR>(group, part_shfl<HEUR>(group, 2));
+    const bool ginternal =
+        pl.sub == 0 && cell_internal<HEUR, WHOLE>(a, OX + (pl.g >> 2) * 4, OY + ((pl.g >> 1) & 1u) * 4, OZ + (pl.g & 1u) * 4, 4,
+                                                  group, group.s02 & 0xFFFFu, group.s13 & 0xFFFFu, group.s02 >> 16,
+                                                  group.s13 >> 16);
+    uint32_t gbits = __ballot_sync(FULL, ginternal);  // bit 4 g
+    gbits = (gbits | (gbits >> 3)) & 0x03030303u;
+    gbits = (gbits | (gbits >> 6)) & 0x000F000Fu;
+    gbits = (gbits | (gbits >> 12)) & 0xFFu;
+    part_merge<HEUR>(group, part_shfl<HEUR>(group, 4));
+    part_merge<HEUR>(group, part_shfl<HEUR>(group, 8));
+    uint32_t s0 = group.s02 & 0xFFFFu, s2 = group.s02 >> 16, s1 = group.s13 & 0xFFFFu, s3 = group.s13 >> 16;
+    const Part other = part_shfl<HEUR>(group, 16);
+    s0 += other.s02 & 0xFFFFu;
+    s2 += other.s02 >> 16;
+    s1 += other.s13 & 0xFFFFu;
+    s3 += other.s13 >> 16;
+    part_merge<HEUR>(group, other);  // its sums may have wrapped, s0..s3 hold them
+    if (lane == 0) {
+        l3 = cell_internal<HEUR, WHOLE>(a, OX, OY, OZ, 8, group, s0, s1, s2, s3);
+        os.s[0] = s0;
+        os.s[1] = s1;
+        os.s[2] = s2;
+        os.s[3] = s3;
+        if (HEUR == XN_HEUR_CHANNEL_DIFF) {
+            os.mn = group.mn02 | (group.mn13 << 8);
+            os.mx = group.mx02 | (group.mx13 << 8);
+        }
+        os.q = group.q;
+        l1 = nibbles_to_bytes(in[0]) | (nibbles_to_bytes(in[1]) << 4);
+        l2 = gbits;
+    }
+}
+
 // One block per brick: the record, and the brick's size, colour, flags and
 // statistics.
 template <int HEUR, bool VEC>
@@ -325,68 +405,16 @@ __global__ void __launch_bounds__(BT) brick_scan_kernel(const __grid_constant__ 
     __shared__ uint32_t s_l2[8], s_l3[8];
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const Place pl = place_of(lane);
-    const uint32_t oy = warp >> 1, oz = warp & 1u;
-    const uint32_t y = Y + oy * 8 + pl.cy * 2, z = Z + oz * 8 + pl.cz * 2;
+    const uint32_t OY = Y + (warp >> 1) * 8, OZ = Z + (warp & 1u) * 8;
     uint4 q[2][4];
 #pragma unroll
-    for (uint32_t h = 0; h < 2; ++h) load_cells<VEC>(a.g, whole, X + h * 8 + pl.cx * 2, y, z, q[h]);
+    for (uint32_t h = 0; h < 2; ++h)
+        load_cells<VEC>(a.g, whole, X + h * 8 + pl.cx * 2, OY + pl.cy * 2, OZ + pl.cz * 2, q[h]);
 #pragma unroll
     for (uint32_t h = 0; h < 2; ++h) {
         const uint32_t o = h * 4 + warp;
-        const uint32_t x = X + h * 8 + pl.cx * 2;
-        Part group = part_empty<HEUR>();
-        uint32_t in[2];
-#pragma unroll
-        for (uint32_t c = 0; c < 2; ++c) {
-            Part p = part_empty<HEUR>();
-#pragma unroll
-            for (uint32_t k = 0; k < 8; ++k) {
-                const bool valid = whole || (x + 2 * c + (k >> 2) < a.g.dx && y + ((k >> 1) & 1u) < a.g.dy &&
-                                             z + (k & 1u) < a.g.dz);
-                part_add<HEUR>(p, cell_voxel(q[h], c, k), valid);
-            }
-            const bool internal = cell_internal<HEUR>(a, whole, x + 2 * c, y, z, 2, p, p.s02 & 0xFFFFu, p.s13 & 0xFFFFu,
-                                                      p.s02 >> 16, p.s13 >> 16);
-            in[c] = __ballot_sync(FULL, internal);
-            if (c == 0) group = p;
-            else part_merge<HEUR>(group, p);
-        }
-        // groups: the four lanes of one
-        part_merge<HEUR>(group, part_shfl<HEUR>(group, 1));
-        part_merge<HEUR>(group, part_shfl<HEUR>(group, 2));
-        const uint32_t gx = X + h * 8 + (pl.g >> 2) * 4, gy = Y + oy * 8 + ((pl.g >> 1) & 1u) * 4,
-                       gz = Z + oz * 8 + (pl.g & 1u) * 4;
-        const bool ginternal = pl.sub == 0 && cell_internal<HEUR>(a, whole, gx, gy, gz, 4, group, group.s02 & 0xFFFFu,
-                                                                  group.s13 & 0xFFFFu, group.s02 >> 16, group.s13 >> 16);
-        uint32_t gbits = __ballot_sync(FULL, ginternal);  // bit 4 g
-        gbits = (gbits | (gbits >> 3)) & 0x03030303u;
-        gbits = (gbits | (gbits >> 6)) & 0x000F000Fu;
-        gbits = (gbits | (gbits >> 12)) & 0xFFu;
-        part_merge<HEUR>(group, part_shfl<HEUR>(group, 4));
-        part_merge<HEUR>(group, part_shfl<HEUR>(group, 8));
-        uint32_t s0 = group.s02 & 0xFFFFu, s2 = group.s02 >> 16, s1 = group.s13 & 0xFFFFu, s3 = group.s13 >> 16;
-        const Part other = part_shfl<HEUR>(group, 16);
-        s0 += other.s02 & 0xFFFFu;
-        s2 += other.s02 >> 16;
-        s1 += other.s13 & 0xFFFFu;
-        s3 += other.s13 >> 16;
-        part_merge<HEUR>(group, other);  // its sums may have wrapped, s0..s3 hold them
-        if (lane == 0) {
-            const bool ointernal = cell_internal<HEUR>(a, whole, X + h * 8, Y + oy * 8, Z + oz * 8, 8, group, s0, s1, s2, s3);
-            OctantSums& os = s_oct[o];
-            os.s[0] = s0;
-            os.s[1] = s1;
-            os.s[2] = s2;
-            os.s[3] = s3;
-            if (HEUR == XN_HEUR_CHANNEL_DIFF) {
-                os.mn = group.mn02 | (group.mn13 << 8);
-                os.mx = group.mx02 | (group.mx13 << 8);
-            }
-            os.q = group.q;
-            s_l1[o] = nibbles_to_bytes(in[0]) | (nibbles_to_bytes(in[1]) << 4);
-            s_l2[o] = gbits;
-            s_l3[o] = ointernal;
-        }
+        if (whole) scan_octant<HEUR, true>(a, q[h], pl, lane, X + h * 8, OY, OZ, s_oct[o], s_l1[o], s_l2[o], s_l3[o]);
+        else scan_octant<HEUR, false>(a, q[h], pl, lane, X + h * 8, OY, OZ, s_oct[o], s_l1[o], s_l2[o], s_l3[o]);
     }
     __syncthreads();
     if (warp != 0) return;
@@ -407,7 +435,9 @@ __global__ void __launch_bounds__(BT) brick_scan_kernel(const __grid_constant__ 
         for (int c = 0; c < 4; ++c) os.s[c] += __shfl_xor_sync(FULL, os.s[c], m);
     }
     bool internal = false;
-    if (lane == 0) internal = cell_internal<HEUR>(a, whole, X, Y, Z, 16, p, os.s[0], os.s[1], os.s[2], os.s[3]);
+    if (lane == 0)
+        internal = whole ? cell_internal<HEUR, true>(a, X, Y, Z, 16, p, os.s[0], os.s[1], os.s[2], os.s[3])
+                         : cell_internal<HEUR, false>(a, X, Y, Z, 16, p, os.s[0], os.s[1], os.s[2], os.s[3]);
     internal = __shfl_sync(FULL, internal, 0);
     // cells below a leaf do not exist
     const uint32_t l3 = internal ? s_l3[o] : 0u;
@@ -453,6 +483,16 @@ __global__ void __launch_bounds__(BT) brick_scan_kernel(const __grid_constant__ 
 
 // ------------------------------------------------------ levels above bricks ---
 
+// s / n for a quotient of at most 255, without a 64-bit division: the rounded
+// quotient of the rounded operands is off by less than 2^-14, so its integer
+// part is off by one at most.
+__device__ __forceinline__ uint32_t byte_quotient(unsigned long long s, unsigned long long n) {
+    uint32_t q = (uint32_t)__fdiv_rn((float)s, (float)n);
+    if (q * n > s) --q;
+    else if (s - q * n >= n) ++q;
+    return q & 0xFFu;
+}
+
 // One cell of depth d < Lb: statistics, decision and size from its children.
 template <int HEUR>
 __device__ void up_cell(const Levels& a, int d, uint64_t i) {
@@ -495,7 +535,7 @@ __device__ void up_cell(const Levels& a, int d, uint64_t i) {
     const uint64_t n = clamped_count(a.g, ox, oy, oz, e);
     uint32_t avg = 0;
 #pragma unroll
-    for (int c = 0; c < 4; ++c) avg |= (uint32_t)(uint8_t)(s[c] / n) << (8 * c);  // Grid.cpp:126-131,180-186
+    for (int c = 0; c < 4; ++c) avg |= byte_quotient(s[c], n) << (8 * c);  // Grid.cpp:126-131,180-186
     bool split;
     if (HEUR == XN_HEUR_CHANNEL_DIFF) {
         CDStats& out = static_cast<CDStats*>(a.stats)[cell];
@@ -637,20 +677,23 @@ __device__ Found climb(const Levels& a, uint32_t Ni, int d, uint32_t x, uint32_t
 
 __device__ __forceinline__ unsigned long long below64(uint32_t n) { return (1ull << n) - 1ull; }  // n < 64
 
-// The same for a cell of extent 2^j, j = 1, 2 or 3 (depth L - j).
+// A brick and its six neighbours (across face f: 1 + f) as a block holds them.
+struct Near {
+    BrickRec rec[7];
+    unsigned long long start[7];
+};
+
+// The same for a cell of extent 2^j, j = 1, 2 or 3 (depth L - j), in the
+// block's brick (bx, by, bz) or, a step across face f, in its neighbour.
 template <int MODE>
-__device__ Found find_cell(const Levels& a, uint32_t Ni, int j, uint32_t cx, uint32_t cy, uint32_t cz) {
+__device__ Found find_cell(const Levels& a, const Near& near, uint32_t bx0, uint32_t by0, uint32_t bz0, uint32_t Ni,
+                           int j, uint32_t f, uint32_t cx, uint32_t cy, uint32_t cz) {
     const int up = BRICK_LEVELS - j;
     const uint32_t bx = cx >> up, by = cy >> up, bz = cz >> up;
-    const LevelGeom& G = a.geo[a.Lb];
-    unsigned long long st = NONE;
-    uint64_t bi = 0;
-    if (bx < G.bx && by < G.by && bz < G.bz) {
-        bi = index_of(G, bx, by, bz);
-        st = a.start[a.off[a.Lb] + bi];
-    }
+    const uint32_t slot = bx == bx0 && by == by0 && bz == bz0 ? 0u : 1u + f;
+    const unsigned long long st = near.start[slot];
     if (st == NONE) return climb<MODE>(a, Ni, a.Lb - 1, bx >> 1, by >> 1, bz >> 1);
-    const BrickRec& r = a.rec[bi];
+    const BrickRec& r = near.rec[slot];
     const uint32_t top = r.top;
     if (!(top & ROOT_BIT)) return Found{leaf_word<MODE>(Ni, (uint32_t)st, digit_sum(bx, by, bz)), 0, 0};
     const uint32_t ox = cx >> (3 - j), oy = cy >> (3 - j), oz = cz >> (3 - j);
@@ -677,11 +720,13 @@ __device__ Found find_cell(const Levels& a, uint32_t Ni, int j, uint32_t cx, uin
 // extent 2^j at (x, y, z) of its depth.  A rope to nothing is 0 in a node
 // and ROPE_EXIT in a record; bricks and larger cells: j >= BRICK_LEVELS.
 template <int MODE>
-__device__ uint32_t rope_of(const Levels& a, uint32_t Ni, int j, uint32_t f, uint32_t x, uint32_t y, uint32_t z) {
+__device__ uint32_t rope_of(const Levels& a, const Near* near, uint32_t bx, uint32_t by, uint32_t bz, uint32_t Ni, int j,
+                            uint32_t f, uint32_t x, uint32_t y, uint32_t z) {
     const uint32_t step = (f & 1u) ? ~0u : 1u, lim = 1u << (a.L - j);
     const uint32_t nx = x + (f < 2 ? step : 0u), ny = y + ((f >> 1) == 1 ? step : 0u), nz = z + (f >= 4 ? step : 0u);
     if (nx >= lim || ny >= lim || nz >= lim) return MODE == BRICK_NODES ? 0u : ROPE_EXIT;  // outside the octree
-    const Found r = j < BRICK_LEVELS ? find_cell<MODE>(a, Ni, j, nx, ny, nz) : climb<MODE>(a, Ni, a.L - j, nx, ny, nz);
+    const Found r = j < BRICK_LEVELS ? find_cell<MODE>(a, *near, bx, by, bz, Ni, j, f, nx, ny, nz)
+                                     : climb<MODE>(a, Ni, a.L - j, nx, ny, nz);
     if (j != 1 || !r.inner) return r.word;
     // an internal cell of 2^3 voxels as the target itself
     return MODE == BRICK_NODES ? r.base - 8u : (r.base - 7u + digit_sum(nx, ny, nz)) / 7u;
@@ -698,12 +743,12 @@ __device__ __forceinline__ void put_node(uint32_t* nodes, uint64_t idx, const ui
 
 // A leaf's node or record; `word` is its leaf_word.
 template <int MODE, bool ROPES>
-__device__ void put_leaf(const WriteArgs& w, uint32_t Ni, uint32_t word, int j, uint32_t x, uint32_t y, uint32_t z,
-                         uint32_t color) {
+__device__ void put_leaf(const WriteArgs& w, const Near* near, uint32_t bx, uint32_t by, uint32_t bz, uint32_t Ni,
+                         uint32_t word, int j, uint32_t x, uint32_t y, uint32_t z, uint32_t color) {
     if (MODE == BRICK_LEAN) return;
 #pragma unroll 1
     for (uint32_t f = 0; f < 6; ++f) {
-        const uint32_t v = ROPES ? rope_of<MODE>(w.a, Ni, j, f, x, y, z) : MODE == BRICK_NODES ? 0u : ROPE_EXIT;
+        const uint32_t v = ROPES ? rope_of<MODE>(w.a, near, bx, by, bz, Ni, j, f, x, y, z) : MODE == BRICK_NODES ? 0u : ROPE_EXIT;
         if (MODE == BRICK_NODES) w.out.nodes[(uint64_t)word * 10 + f] = v;
         else w.out.leaves[(uint64_t)(word & ~LEAF) * 8 + 1 + f] = v;
     }
@@ -742,9 +787,8 @@ __device__ __forceinline__ void put_inner(const WriteArgs& w, uint32_t rank, uin
 
 // The cells of depth Lb and above: leaves, and internal nodes above the bricks.
 template <int MODE, bool ROPES>
-__global__ void __launch_bounds__(128) coarse_write_kernel(const __grid_constant__ WriteArgs w) {
+__device__ void write_coarse(const WriteArgs& w, uint64_t c) {
     const Levels& a = w.a;
-    const uint64_t c = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= a.off[a.Lb + 1]) return;
     const unsigned long long st = a.start[c];
     if (st == NONE) return;
@@ -758,7 +802,7 @@ __global__ void __launch_bounds__(128) coarse_write_kernel(const __grid_constant
     coords_of(c - a.off[d], a.geo[d], x, y, z);
     const uint32_t P = digit_sum(x, y, z);
     if (fl & F_LEAF) {
-        put_leaf<MODE, ROPES>(w, Ni, leaf_word<MODE>(Ni, (uint32_t)st, P), a.L - d, x, y, z, a.color[c]);
+        put_leaf<MODE, ROPES>(w, nullptr, 0, 0, 0, Ni, leaf_word<MODE>(Ni, (uint32_t)st, P), a.L - d, x, y, z, a.color[c]);
         return;
     }
     const uint32_t rank = Ni - (uint32_t)st - (uint32_t)a.size[c];
@@ -790,11 +834,18 @@ struct StageOf { using T = VoxelStage; };
 template <>
 struct StageOf<false> { using T = NoStage; };
 
-// One block per brick that is internal: its internal nodes and their leaves.
+// One block per brick that is internal, a warp per octant: its internal nodes
+// and their leaves.  The blocks after the bricks' write the cells above, a
+// thread each.
+constexpr int WT = 256;
 template <int MODE, bool ROPES, bool VEC>
-__global__ void __launch_bounds__(BT) brick_write_kernel(const __grid_constant__ WriteArgs w) {
+__global__ void __launch_bounds__(WT) brick_write_kernel(const __grid_constant__ WriteArgs w) {
     const Levels& a = w.a;
     const uint64_t b = blockIdx.x;
+    if (b >= a.geo[a.Lb].n) {
+        write_coarse<MODE, ROPES>(w, (b - a.geo[a.Lb].n) * WT + threadIdx.x);
+        return;
+    }
     const unsigned long long st = a.start[a.off[a.Lb] + b];
     const BrickRec& rec = a.rec[b];
     const uint32_t top = rec.top;
@@ -811,204 +862,218 @@ __global__ void __launch_bounds__(BT) brick_write_kernel(const __grid_constant__
     const uint32_t Pb = digit_sum(bx, by, bz);
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const Place pl = place_of(lane);
-    const uint32_t oy = warp >> 1, oz = warp & 1u;
+    const uint32_t o = warp, h = o >> 2, oy = (o >> 1) & 1u, oz = o & 1u;
     constexpr bool STAGED = MODE != BRICK_LEAN;
-    __shared__ typename StageOf<STAGED>::T s_stage[STAGED ? BT / 32 : 1];
-    __shared__ __align__(16) uint32_t s_nodes[MODE == BRICK_NODES ? BT / 32 : 1][MODE == BRICK_NODES ? 320 : 1];
+    __shared__ typename StageOf<STAGED>::T s_stage[STAGED ? WT / 32 : 1];
+    __shared__ __align__(16) uint32_t s_nodes[MODE == BRICK_NODES ? WT / 32 : 1][MODE == BRICK_NODES ? 320 : 1];
     if (threadIdx.x == 0) put_inner<MODE>(w, brank, Pb, a.color[a.off[a.Lb] + b], a.Lb);
-#pragma unroll 1
-    for (uint32_t h = 0; h < 2; ++h) {
-        const uint32_t o = h * 4 + warp;
-        const uint32_t so = bsi + rec.pre[o];
-        const uint32_t Ox = bx * 2 + h, Oy = by * 2 + oy, Oz = bz * 2 + oz;  // octant coordinates (depth L - 3)
-        const uint32_t Po = Pb + o;
-        if (!(top >> o & 1u)) {
-            if (lane == 0) {
-                const uint32_t word = leaf_word<MODE>(Ni, so, Po);
-                put_child<MODE>(w, brank, Pb, o, false, word, rec.ocol[o]);
-                put_leaf<MODE, ROPES>(w, Ni, word, 3, Ox, Oy, Oz, rec.ocol[o]);
-            }
-            continue;
+    __shared__ Near s_near;
+    if (ROPES) {  // the records that ropes can reach
+        if (threadIdx.x < 7) {
+            const uint32_t f = threadIdx.x - 1u, step = (f & 1u) ? ~0u : 1u;
+            const uint32_t nx = bx + (threadIdx.x && f < 2 ? step : 0u), ny = by + (threadIdx.x && (f >> 1) == 1 ? step : 0u),
+                           nz = bz + (threadIdx.x && f >= 4 ? step : 0u);
+            s_near.start[threadIdx.x] =
+                nx < G.bx && ny < G.by && nz < G.bz ? a.start[a.off[a.Lb] + index_of(G, nx, ny, nz)] : NONE;
         }
-        const unsigned long long l1 = rec.l1[o];
-        const uint32_t l2 = (uint32_t)(rec.l2 >> (8 * o)) & 0xFFu;
-        uint4 q[4];
-        load_cells<VEC>(a.g, whole, X + h * 8 + pl.cx * 2, Y + oy * 8 + pl.cy * 2, Z + oz * 8 + pl.cz * 2, q);
-        const uint32_t orank = Ni - so - (__popcll(l1) + __popc(l2) + 1u);
-        const uint32_t g = pl.g;
-        const uint32_t cells = (uint32_t)(l1 >> (8 * g)) & 0xFFu;  // the group's internal cells
-        const bool ginternal = l2 >> g & 1u;
-        const uint32_t sg = so + __popcll(l1 & below64(8 * g)) + __popc(l2 & ((1u << g) - 1u));
-        const uint32_t Gx = Ox * 2 + (g >> 2), Gy = Oy * 2 + ((g >> 1) & 1u), Gz = Oz * 2 + (g & 1u);
-        const uint32_t Pg = Po + g;
-        const uint32_t grank = Ni - sg - (__popc(cells) + 1u);
-        // sums: of the lane's two cells, its group and the octant
-        uint32_t c02[2], c13[2];
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < 7 * sizeof(BrickRec) / 16; i += WT) {
+            const uint32_t slot = i / (sizeof(BrickRec) / 16), f = slot - 1u, step = (f & 1u) ? ~0u : 1u;
+            if (s_near.start[slot] == NONE) continue;
+            const uint64_t bi = index_of(G, bx + (slot && f < 2 ? step : 0u), by + (slot && (f >> 1) == 1 ? step : 0u),
+                                         bz + (slot && f >= 4 ? step : 0u));
+            reinterpret_cast<uint4*>(s_near.rec)[i] = reinterpret_cast<const uint4*>(a.rec + bi)[i % (sizeof(BrickRec) / 16)];
+        }
+        __syncthreads();
+    }
+    const uint32_t so = bsi + rec.pre[o];
+    const uint32_t Ox = bx * 2 + h, Oy = by * 2 + oy, Oz = bz * 2 + oz;  // octant coordinates (depth L - 3)
+    const uint32_t Po = Pb + o;
+    if (!(top >> o & 1u)) {
+        if (lane == 0) {
+            const uint32_t word = leaf_word<MODE>(Ni, so, Po);
+            put_child<MODE>(w, brank, Pb, o, false, word, rec.ocol[o]);
+            put_leaf<MODE, ROPES>(w, &s_near, bx, by, bz, Ni, word, 3, Ox, Oy, Oz, rec.ocol[o]);
+        }
+        return;
+    }
+    const unsigned long long l1 = rec.l1[o];
+    const uint32_t l2 = (uint32_t)(rec.l2 >> (8 * o)) & 0xFFu;
+    uint4 q[4];
+    load_cells<VEC>(a.g, whole, X + h * 8 + pl.cx * 2, Y + oy * 8 + pl.cy * 2, Z + oz * 8 + pl.cz * 2, q);
+    const uint32_t orank = Ni - so - (__popcll(l1) + __popc(l2) + 1u);
+    const uint32_t g = pl.g;
+    const uint32_t cells = (uint32_t)(l1 >> (8 * g)) & 0xFFu;  // the group's internal cells
+    const bool ginternal = l2 >> g & 1u;
+    const uint32_t sg = so + __popcll(l1 & below64(8 * g)) + __popc(l2 & ((1u << g) - 1u));
+    const uint32_t Gx = Ox * 2 + (g >> 2), Gy = Oy * 2 + ((g >> 1) & 1u), Gz = Oz * 2 + (g & 1u);
+    const uint32_t Pg = Po + g;
+    const uint32_t grank = Ni - sg - (__popc(cells) + 1u);
+    // sums: of the lane's two cells, its group and the octant
+    uint32_t c02[2], c13[2];
+#pragma unroll
+    for (uint32_t c = 0; c < 2; ++c) {
+        c02[c] = c13[c] = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; ++k) {
+            const uint32_t v = cell_voxel(q, c, k);
+            c02[c] += v & 0x00FF00FFu;
+            c13[c] += (v >> 8) & 0x00FF00FFu;
+        }
+    }
+    uint32_t g02 = c02[0] + c02[1], g13 = c13[0] + c13[1];
+    g02 += __shfl_xor_sync(FULL, g02, 1);
+    g13 += __shfl_xor_sync(FULL, g13, 1);
+    g02 += __shfl_xor_sync(FULL, g02, 2);
+    g13 += __shfl_xor_sync(FULL, g13, 2);
+    // a leaf cell is whole or outside the grid (all zeros), so its average
+    // is a shift; only a partly covered internal node divides
+    uint32_t gcol = ((g02 >> 6) & 0x00FF00FFu) | (((g13 >> 6) & 0x00FF00FFu) << 8);
+    if (MODE == BRICK_NODES && !whole && ginternal) {
+        const uint32_t n = count_in(a.g, Gx * 4, Gy * 4, Gz * 4, 4);
+        gcol = average4(g02 & 0xFFFFu, g13 & 0xFFFFu, g02 >> 16, g13 >> 16, n);
+    }
+    if (lane == 0) {
+        put_child<MODE>(w, brank, Pb, o, true, inner_word<MODE>(orank, Po), 0);
+        put_inner<MODE>(w, orank, Po, MODE == BRICK_NODES ? rec.ocol[o] : 0u, a.L - 3);
+    }
+    if (pl.sub == 0) {
+        const uint32_t word = ginternal ? inner_word<MODE>(grank, Pg) : leaf_word<MODE>(Ni, sg, Pg);
+        put_child<MODE>(w, orank, Po, g, ginternal, word, gcol);
+        if (ginternal) put_inner<MODE>(w, grank, Pg, gcol, a.L - 2);
+        else put_leaf<MODE, ROPES>(w, &s_near, bx, by, bz, Ni, word, 2, Gx, Gy, Gz, gcol);
+    }
+    if (ginternal) {
 #pragma unroll
         for (uint32_t c = 0; c < 2; ++c) {
-            c02[c] = c13[c] = 0;
-#pragma unroll
-            for (uint32_t k = 0; k < 8; ++k) {
-                const uint32_t v = cell_voxel(q, c, k);
-                c02[c] += v & 0x00FF00FFu;
-                c13[c] += (v >> 8) & 0x00FF00FFu;
+            const uint32_t k = c * 4 + pl.sub;
+            const uint32_t m = g * 8 + k;
+            const bool internal = cells >> k & 1u;
+            const uint32_t sc = sg + __popc(cells & ((1u << k) - 1u));
+            const uint32_t Pc = Pg + k;
+            const uint32_t Cx = Gx * 2 + c, Cy = Gy * 2 + (pl.sub >> 1), Cz = Gz * 2 + (pl.sub & 1u);
+            uint32_t col = ((c02[c] >> 3) & 0x00FF00FFu) | (((c13[c] >> 3) & 0x00FF00FFu) << 8);
+            const uint32_t rank = Ni - sc - 1u;
+            const uint32_t word = internal ? inner_word<MODE>(rank, Pc) : leaf_word<MODE>(Ni, sc, Pc);
+            put_child<MODE>(w, grank, Pg, k, internal, word, col);
+            if (!internal) {
+                put_leaf<MODE, ROPES>(w, &s_near, bx, by, bz, Ni, word, 1, Cx, Cy, Cz, col);
+                continue;
             }
-        }
-        uint32_t g02 = c02[0] + c02[1], g13 = c13[0] + c13[1];
-        g02 += __shfl_xor_sync(FULL, g02, 1);
-        g13 += __shfl_xor_sync(FULL, g13, 1);
-        g02 += __shfl_xor_sync(FULL, g02, 2);
-        g13 += __shfl_xor_sync(FULL, g13, 2);
-        // a leaf cell is whole or outside the grid (all zeros), so its average
-        // is a shift; only a partly covered internal node divides
-        uint32_t gcol = ((g02 >> 6) & 0x00FF00FFu) | (((g13 >> 6) & 0x00FF00FFu) << 8);
-        if (MODE == BRICK_NODES && !whole && ginternal) {
-            const uint32_t n = count_in(a.g, Gx * 4, Gy * 4, Gz * 4, 4);
-            gcol = average4(g02 & 0xFFFFu, g13 & 0xFFFFu, g02 >> 16, g13 >> 16, n);
-        }
-        if (lane == 0) {
-            put_child<MODE>(w, brank, Pb, o, true, inner_word<MODE>(orank, Po), 0);
-            put_inner<MODE>(w, orank, Po, MODE == BRICK_NODES ? rec.ocol[o] : 0u, a.L - 3);
-        }
-        if (pl.sub == 0) {
-            const uint32_t word = ginternal ? inner_word<MODE>(grank, Pg) : leaf_word<MODE>(Ni, sg, Pg);
-            put_child<MODE>(w, orank, Po, g, ginternal, word, gcol);
-            if (ginternal) put_inner<MODE>(w, grank, Pg, gcol, a.L - 2);
-            else put_leaf<MODE, ROPES>(w, Ni, word, 2, Gx, Gy, Gz, gcol);
-        }
-        if (ginternal) {
+            uint32_t v[8];
 #pragma unroll
-            for (uint32_t c = 0; c < 2; ++c) {
-                const uint32_t k = c * 4 + pl.sub;
-                const uint32_t m = g * 8 + k;
-                const bool internal = cells >> k & 1u;
-                const uint32_t sc = sg + __popc(cells & ((1u << k) - 1u));
-                const uint32_t Pc = Pg + k;
-                const uint32_t Cx = Gx * 2 + c, Cy = Gy * 2 + (pl.sub >> 1), Cz = Gz * 2 + (pl.sub & 1u);
-                uint32_t col = ((c02[c] >> 3) & 0x00FF00FFu) | (((c13[c] >> 3) & 0x00FF00FFu) << 8);
-                const uint32_t rank = Ni - sc - 1u;
-                const uint32_t word = internal ? inner_word<MODE>(rank, Pc) : leaf_word<MODE>(Ni, sc, Pc);
-                put_child<MODE>(w, grank, Pg, k, internal, word, col);
-                if (!internal) {
-                    put_leaf<MODE, ROPES>(w, Ni, word, 1, Cx, Cy, Cz, col);
-                    continue;
+            for (uint32_t t = 0; t < 8; ++t) v[t] = cell_voxel(q, c, t);
+            const uint32_t base = (MODE == BRICK_NODES ? 8u : 7u) * (Ni - sc) - Pc;
+            if constexpr (MODE == BRICK_NODES) {
+                if (!whole) {
+                    const uint32_t n = count_in(a.g, Cx * 2, Cy * 2, Cz * 2, 2);
+                    col = average4(c02[c] & 0xFFFFu, c13[c] & 0xFFFFu, c02[c] >> 16, c13[c] >> 16, n);
                 }
-                uint32_t v[8];
+                uint32_t ch[8];
 #pragma unroll
-                for (uint32_t t = 0; t < 8; ++t) v[t] = cell_voxel(q, c, t);
-                const uint32_t base = (MODE == BRICK_NODES ? 8u : 7u) * (Ni - sc) - Pc;
-                if constexpr (MODE == BRICK_NODES) {
-                    if (!whole) {
-                        const uint32_t n = count_in(a.g, Cx * 2, Cy * 2, Cz * 2, 2);
-                        col = average4(c02[c] & 0xFFFFu, c13[c] & 0xFFFFu, c02[c] >> 16, c13[c] >> 16, n);
-                    }
-                    uint32_t ch[8];
-#pragma unroll
-                    for (uint32_t t = 0; t < 8; ++t) ch[t] = base - t;
-                    put_node(w.out.nodes, 8u * rank - Pc, ch, col, (uint32_t)(a.L - 1 + w.depth_off));
-                } else {
-                    uint4* p = reinterpret_cast<uint4*>(w.out.inner + (uint64_t)rank * 8);
-                    p[0] = make_uint4(LEAF | (v[0] & 0xFFFFFFu), LEAF | (v[1] & 0xFFFFFFu), LEAF | (v[2] & 0xFFFFFFu),
-                                      LEAF | (v[3] & 0xFFFFFFu));
-                    p[1] = make_uint4(LEAF | (v[4] & 0xFFFFFFu), LEAF | (v[5] & 0xFFFFFFu), LEAF | (v[6] & 0xFFFFFFu),
-                                      LEAF | (v[7] & 0xFFFFFFu));
-                    w.out.inner_depth[rank] = (uint32_t)(a.L - 1);
-                    if constexpr (MODE == BRICK_LAYOUT) {
-                        uint4* p2 = reinterpret_cast<uint4*>(w.out.rinner + (uint64_t)rank * 8);
-                        p2[0] = make_uint4(LEAF | base, LEAF | (base - 1), LEAF | (base - 2), LEAF | (base - 3));
-                        p2[1] = make_uint4(LEAF | (base - 4), LEAF | (base - 5), LEAF | (base - 6), LEAF | (base - 7));
-                    }
-                }
-                if constexpr (STAGED) {
-                    VoxelStage& sg_ = s_stage[warp];
-#pragma unroll
-                    for (uint32_t t = 0; t < 8; ++t) sg_.vox[m][t] = v[t];
-                    sg_.base[m] = base;
-                    sg_.list[__popcll(l1 & below64(m))] = (uint8_t)m;
-                    if constexpr (ROPES) {
-                        uint32_t fine = 0;
-                        const uint32_t lim = 1u << (a.L - 1);
-#pragma unroll 1
-                        for (uint32_t f = 0; f < 6; ++f) {
-                            const uint32_t step = (f & 1u) ? ~0u : 1u;
-                            const uint32_t nx = Cx + (f < 2 ? step : 0u), ny = Cy + ((f >> 1) == 1 ? step : 0u),
-                                           nz = Cz + (f >= 4 ? step : 0u);
-                            uint32_t word2 = MODE == BRICK_NODES ? 0u : ROPE_EXIT;
-                            if (nx < lim && ny < lim && nz < lim) {
-                                const Found r = find_cell<MODE>(a, Ni, 1, nx, ny, nz);
-                                word2 = r.inner ? r.base : r.word;
-                                fine |= r.inner << f;
-                            }
-                            sg_.face[m][f] = word2;
-                        }
-                        sg_.fine[m] = (uint8_t)fine;
-                    }
-                }
-            }
-        }
-        if constexpr (STAGED) {
-            VoxelStage& sg_ = s_stage[warp];
-            __syncwarp();
-            const uint32_t total = 8u * __popcll(l1);
-            for (uint32_t t0 = 0; t0 < total; t0 += 32) {
-                const uint32_t t = t0 + lane;
-                const bool on = t < total;
-                const uint32_t m = on ? sg_.list[t >> 3] : 0u, k = t & 7u;
-                uint32_t r[6];
-                uint32_t idx = 0, color = 0;
-                if (on) {
-                    idx = sg_.base[m] - k;
-                    color = sg_.vox[m][k];
-                    if (ROPES) {
-                        const uint32_t fine = sg_.fine[m];
-#pragma unroll
-                        for (uint32_t f = 0; f < 6; ++f) {
-                            const uint32_t bit = 4u >> (f >> 1);
-                            // towards +axis the sibling is the child with the
-                            // axis bit set, towards -axis the one without
-                            const bool sibling = ((k & bit) != 0) == ((f & 1u) != 0);
-                            const uint32_t kn = k ^ bit;
-                            const uint32_t face = sg_.face[m][f];
-                            const uint32_t target = (sibling ? sg_.base[m] : face) - kn;
-                            r[f] = sibling || (fine >> f & 1u) ? (MODE == BRICK_NODES ? target : LEAF | target) : face;
-                        }
-                    } else {
-#pragma unroll
-                        for (uint32_t f = 0; f < 6; ++f) r[f] = MODE == BRICK_NODES ? 0u : ROPE_EXIT;
-                    }
-                }
-                const uint32_t depth = LEAF | (uint32_t)(a.L + w.depth_off);
+                for (uint32_t t = 0; t < 8; ++t) ch[t] = base - t;
+                put_node(w.out.nodes, 8u * rank - Pc, ch, col, (uint32_t)(a.L - 1 + w.depth_off));
+            } else {
+                uint4* p = reinterpret_cast<uint4*>(w.out.inner + (uint64_t)rank * 8);
+                p[0] = make_uint4(LEAF | (v[0] & 0xFFFFFFu), LEAF | (v[1] & 0xFFFFFFu), LEAF | (v[2] & 0xFFFFFFu),
+                                  LEAF | (v[3] & 0xFFFFFFu));
+                p[1] = make_uint4(LEAF | (v[4] & 0xFFFFFFu), LEAF | (v[5] & 0xFFFFFFu), LEAF | (v[6] & 0xFFFFFFu),
+                                  LEAF | (v[7] & 0xFFFFFFu));
+                w.out.inner_depth[rank] = (uint32_t)(a.L - 1);
                 if constexpr (MODE == BRICK_LAYOUT) {
-                    if (on) {
-                        uint4* p = reinterpret_cast<uint4*>(w.out.leaves + (uint64_t)idx * 8);
-                        p[0] = make_uint4(color, r[0], r[1], r[2]);
-                        p[1] = make_uint4(r[3], r[4], r[5], depth);
-                    }
-                } else {
-                    // through shared memory, so that neighbouring lanes write
-                    // neighbouring words of the 40-byte nodes
-                    uint32_t* sn = s_nodes[warp];
-                    if (on) {
-                        uint2* p = reinterpret_cast<uint2*>(sn + lane * 10);
-                        p[0] = make_uint2(r[0], r[1]);
-                        p[1] = make_uint2(r[2], r[3]);
-                        p[2] = make_uint2(r[4], r[5]);
-                        p[3] = make_uint2(0, 0);
-                        p[4] = make_uint2(color, depth);
-                    }
-                    __syncwarp();
-                    const uint32_t words = min(32u, total - t0) * 10u;
-#pragma unroll
-                    for (uint32_t i = 0; i < 10; ++i) {
-                        const uint32_t wd = i * 32 + lane;
-                        const uint32_t node = wd / 10u;
-                        const uint32_t at = __shfl_sync(FULL, idx, node & 31u);
-                        if (wd < words) w.out.nodes[(uint64_t)at * 10 + (wd - node * 10u)] = sn[wd];
-                    }
-                    __syncwarp();
+                    uint4* p2 = reinterpret_cast<uint4*>(w.out.rinner + (uint64_t)rank * 8);
+                    p2[0] = make_uint4(LEAF | base, LEAF | (base - 1), LEAF | (base - 2), LEAF | (base - 3));
+                    p2[1] = make_uint4(LEAF | (base - 4), LEAF | (base - 5), LEAF | (base - 6), LEAF | (base - 7));
                 }
             }
-            __syncwarp();  // the stage is used again by the warp's other octant
+            if constexpr (STAGED) {
+                VoxelStage& sg_ = s_stage[warp];
+#pragma unroll
+                for (uint32_t t = 0; t < 8; ++t) sg_.vox[m][t] = v[t];
+                sg_.base[m] = base;
+                sg_.list[__popcll(l1 & below64(m))] = (uint8_t)m;
+                if constexpr (ROPES) {
+                    uint32_t fine = 0;
+                    const uint32_t lim = 1u << (a.L - 1);
+#pragma unroll 1
+                    for (uint32_t f = 0; f < 6; ++f) {
+                        const uint32_t step = (f & 1u) ? ~0u : 1u;
+                        const uint32_t nx = Cx + (f < 2 ? step : 0u), ny = Cy + ((f >> 1) == 1 ? step : 0u),
+                                       nz = Cz + (f >= 4 ? step : 0u);
+                        uint32_t word2 = MODE == BRICK_NODES ? 0u : ROPE_EXIT;
+                        if (nx < lim && ny < lim && nz < lim) {
+                            const Found r = find_cell<MODE>(a, s_near, bx, by, bz, Ni, 1, f, nx, ny, nz);
+                            word2 = r.inner ? r.base : r.word;
+                            fine |= r.inner << f;
+                        }
+                        sg_.face[m][f] = word2;
+                    }
+                    sg_.fine[m] = (uint8_t)fine;
+                }
+            }
+        }
+    }
+    if constexpr (STAGED) {
+        VoxelStage& sg_ = s_stage[warp];
+        __syncwarp();
+        const uint32_t total = 8u * __popcll(l1);
+        for (uint32_t t0 = 0; t0 < total; t0 += 32) {
+            const uint32_t t = t0 + lane;
+            const bool on = t < total;
+            const uint32_t m = on ? sg_.list[t >> 3] : 0u, k = t & 7u;
+            uint32_t r[6];
+            uint32_t idx = 0, color = 0;
+            if (on) {
+                idx = sg_.base[m] - k;
+                color = sg_.vox[m][k];
+                if (ROPES) {
+                    const uint32_t fine = sg_.fine[m];
+#pragma unroll
+                    for (uint32_t f = 0; f < 6; ++f) {
+                        const uint32_t bit = 4u >> (f >> 1);
+                        // towards +axis the sibling is the child with the
+                        // axis bit set, towards -axis the one without
+                        const bool sibling = ((k & bit) != 0) == ((f & 1u) != 0);
+                        const uint32_t kn = k ^ bit;
+                        const uint32_t face = sg_.face[m][f];
+                        const uint32_t target = (sibling ? sg_.base[m] : face) - kn;
+                        r[f] = sibling || (fine >> f & 1u) ? (MODE == BRICK_NODES ? target : LEAF | target) : face;
+                    }
+                } else {
+#pragma unroll
+                    for (uint32_t f = 0; f < 6; ++f) r[f] = MODE == BRICK_NODES ? 0u : ROPE_EXIT;
+                }
+            }
+            const uint32_t depth = LEAF | (uint32_t)(a.L + w.depth_off);
+            if constexpr (MODE == BRICK_LAYOUT) {
+                if (on) {
+                    uint4* p = reinterpret_cast<uint4*>(w.out.leaves + (uint64_t)idx * 8);
+                    p[0] = make_uint4(color, r[0], r[1], r[2]);
+                    p[1] = make_uint4(r[3], r[4], r[5], depth);
+                }
+            } else {
+                // through shared memory, so that neighbouring lanes write
+                // neighbouring words of the 40-byte nodes
+                uint32_t* sn = s_nodes[warp];
+                if (on) {
+                    uint2* p = reinterpret_cast<uint2*>(sn + lane * 10);
+                    p[0] = make_uint2(r[0], r[1]);
+                    p[1] = make_uint2(r[2], r[3]);
+                    p[2] = make_uint2(r[4], r[5]);
+                    p[3] = make_uint2(0, 0);
+                    p[4] = make_uint2(color, depth);
+                }
+                __syncwarp();
+                const uint32_t words = min(32u, total - t0) * 10u;
+#pragma unroll
+                for (uint32_t i = 0; i < 10; ++i) {
+                    const uint32_t wd = i * 32 + lane;
+                    const uint32_t node = wd / 10u;
+                    const uint32_t at = __shfl_sync(FULL, idx, node & 31u);
+                    if (wd < words) w.out.nodes[(uint64_t)at * 10 + (wd - node * 10u)] = sn[wd];
+                }
+                __syncwarp();
+            }
         }
     }
 }
@@ -1019,10 +1084,9 @@ bool vector_rows(const GridDev& g) { return g.dx % 4 == 0 && (reinterpret_cast<u
 
 template <int MODE, bool ROPES>
 void launch_write(const WriteArgs& w, cudaStream_t s) {
-    coarse_write_kernel<MODE, ROPES><<<blocks_for(w.a.off[w.a.Lb + 1], 128), 128, 0, s>>>(w);
-    const unsigned nb = (unsigned)w.a.geo[w.a.Lb].n;
-    if (vector_rows(w.a.g)) brick_write_kernel<MODE, ROPES, true><<<nb, BT, 0, s>>>(w);
-    else brick_write_kernel<MODE, ROPES, false><<<nb, BT, 0, s>>>(w);
+    const unsigned nb = (unsigned)w.a.geo[w.a.Lb].n + blocks_for(w.a.off[w.a.Lb + 1], WT);
+    if (vector_rows(w.a.g)) brick_write_kernel<MODE, ROPES, true><<<nb, WT, 0, s>>>(w);
+    else brick_write_kernel<MODE, ROPES, false><<<nb, WT, 0, s>>>(w);
 }
 
 }  // namespace

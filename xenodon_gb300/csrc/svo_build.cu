@@ -611,7 +611,7 @@ int build_bricks(Ctx* c, const GridDev& g, uint64_t side, int L, bool ropes, int
     b.stddev = threshold;
     b.sequential = heuristic == XN_HEUR_STD_DEV && getenv("XN_BUILD_STDDEV_SEQUENTIAL") != nullptr;
     const uint64_t bytes = brick_plan(b, side, nullptr);
-    if (b.geo[b.Lb].n > 0x7FFFFFFFull) return fail(XN_ERR_ARG, "xn_build_svo: grid too large");
+    if (b.off[b.Lb + 1] > 0x70000000ull) return fail(XN_ERR_ARG, "xn_build_svo: grid too large");
     unsigned char* base = nullptr;
     int r;
     if ((r = sc.alloc(&base, bytes, "xn_build_svo: scratch"))) return r;
