@@ -99,6 +99,7 @@ struct Request {
 // Buffers of power-of-two sizes, kept for reuse (device or pinned host).
 struct Pool {
     bool device = true;
+    xn::Ctx* ctx = nullptr;  // of a device pool
     std::multimap<uint64_t, void*> free;
     std::vector<std::pair<void*, uint64_t>> all;
     static uint64_t round(uint64_t b) {
@@ -116,7 +117,12 @@ struct Pool {
             return p;
         }
         void* p = nullptr;
-        const cudaError_t e = device ? cudaMalloc(&p, r) : cudaHostAlloc(&p, r, cudaHostAllocDefault);
+        cudaError_t e = device ? cudaMalloc(&p, r) : cudaHostAlloc(&p, r, cudaHostAllocDefault);
+        if (device && e == cudaErrorMemoryAllocation) {  // the context's freed blocks may be in the way
+            cudaGetLastError();
+            ctx->trim_pool(0);
+            e = cudaMalloc(&p, r);
+        }
         if (e != cudaSuccess) return nullptr;
         all.emplace_back(p, r);
         *got = r;
@@ -655,6 +661,7 @@ XN_API int xn_server_create(xn_ctx* ctx, const xn_server_config* cfg, xn_server*
     if (s->cfg.fold_blocks_per_sm == 0) s->cfg.fold_blocks_per_sm = 2;
     if (s->cfg.fold_blocks_per_sm > 4) s->cfg.fold_blocks_per_sm = 4;
     s->host_pool.device = false;
+    s->dev_pool.ctx = s->c;
     if (const char* tp = std::getenv("XN_SERVER_TRACE")) s->trace_path = tp;
     if (const char* ft = std::getenv("XN_FOLD_THREADS")) s->fold_threads = std::atoi(ft) == 32 ? 32u : 128u;
     uint64_t used = 0, budget = 0;
