@@ -129,9 +129,23 @@ __device__ __forceinline__ V3 tex_texel(cudaTextureObject_t t, float x, float y,
     return V3{s_unorm_lut[v.x], s_unorm_lut[v.y], s_unorm_lut[v.z]};
 }
 
-// resources/dda.comp:13-53 over the texture form; coordinates are kept as
-// texel centres (integers + 0.5, exact in float).
-template <bool COUNT, int NORM>
+// resources/dda.comp:13-53 over the texture form; coordinates are kept as texel
+// centres (integers + 0.5, exact in float).  The steps do not depend on the
+// texels, so a round makes DDA_AHEAD steps and fetches and then adds their
+// products in order: that many fetches of a ray are in flight, and the loop's
+// own work is shared by them.  A round that reaches the ray's end adds only the
+// steps before it; the fetches past it read texels the sum never uses (in range
+// or the zero border).  Mrays/s with one fetch ahead, and with rounds of 4 and 8
+// (32, 46 and 47 registers): 128^3 blobs at 256x256 1221, 2659, 2755; at 512x512 4817,
+// 7450, 7609; at 1920x1080 8464, 9337, 9282; 512^3 gas field at 256x256 117, 350,
+// 365; 1024^3 at 3840x2160, where the texture unit is the bound, 925, 943, 952.
+// Held to 32 registers (16 blocks an SM), rounds of 4 gave 1245 and 939 of these.
+// In the batch kernel, whose many frames fill the GPU, rounds of 2 in 32 registers
+// are the best: 40 frames of 256x256 of a 400^3 gas field 2651 us with one fetch
+// ahead, 2277 with rounds of 2, 2933 of 4 and (64 registers) 2927 of 4, 3100 of 8;
+// of 128^3 blobs 640, 426, 704, 480, 495.
+constexpr int DDA_AHEAD = 8, DDA_AHEAD_BATCH = 2;
+template <bool COUNT, int NORM, int K = DDA_AHEAD>
 __device__ V3 trace_dda_tex(cudaTextureObject_t tex, uint32_t dx, uint32_t dy, uint32_t dz, V3 ro, V3 rd,
                             uint32_t& loads, uint32_t& err) {
     V3 rrd = vs(1.0f) / rd;
@@ -152,26 +166,33 @@ __device__ V3 trace_dda_tex(cudaTextureObject_t tex, uint32_t dx, uint32_t dy, u
     float t = 0.0f;
     V3 total = vs(0.0f);
     const float lim = t_max - t_min;
-    const uint32_t cap = 2u * (dx + dy + dz) + 64u;
+    const uint32_t cap = (2u * (dx + dy + dz) + 64u) / K + 1u;
     uint32_t iter = 0;
-    // The texel of the next step does not depend on this one's value: fetch
-    // it before accumulating the current one so the texture latency overlaps
-    // the step arithmetic.  The fetch after the last step reads a texel the
-    // sum never uses (in range or the zero border).
-    V3 tx = tex_texel<NORM>(tex, px, py, pz);
     while (t < lim) {
         if (++iter > cap) { err |= 1u; break; }
-        if (COUNT) ++loads;
-        // lessThanEqual(side, min(side.yzx, side.zxy)) is side.k == min of
-        // all three (the sides are finite and positive)
-        const float t0 = min3f(side.x, side.y, side.z);
-        if (side.x == t0) { side.x = side.x + t_delta.x; px += sgn.x; }
-        if (side.y == t0) { side.y = side.y + t_delta.y; py += sgn.y; }
-        if (side.z == t0) { side.z = side.z + t_delta.z; pz += sgn.z; }
-        const V3 next = tex_texel<NORM>(tex, px, py, pz);
-        total = total + tx * (t0 - t);
-        t = t0;
-        tx = next;
+        V3 c[K];
+        float ts[K];  // where each step starts
+        float dt[K];
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            c[i] = tex_texel<NORM>(tex, px, py, pz);
+            // lessThanEqual(side, min(side.yzx, side.zxy)) is side.k == min of
+            // all three (the sides are finite and positive)
+            const float t0 = min3f(side.x, side.y, side.z);
+            if (side.x == t0) { side.x = side.x + t_delta.x; px += sgn.x; }
+            if (side.y == t0) { side.y = side.y + t_delta.y; py += sgn.y; }
+            if (side.z == t0) { side.z = side.z + t_delta.z; pz += sgn.z; }
+            ts[i] = t;
+            dt[i] = t0 - t;
+            t = t0;
+        }
+#pragma unroll
+        for (int i = 0; i < K; ++i) {
+            if (i == 0 || ts[i] < lim) {
+                total = total + c[i] * dt[i];
+                if (COUNT) ++loads;
+            }
+        }
     }
     return total;
 }
@@ -1997,11 +2018,11 @@ __device__ __forceinline__ uint32_t render_job_pixel_spec(const BatchJob& J, uin
             const V3 ro = f.translation * side;
             const float ec = __fdiv_rn(voxel_emission_coeff(f, rd), side);
             if (SPEC == XN_BATCH_DDA_TEX_NORM)
-                color = trace_dda_tex<false, TEX_NORM>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err) * ec;
+                color = trace_dda_tex<false, TEX_NORM, DDA_AHEAD_BATCH>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err) * ec;
             else if (J.tex_normalized == TEX_PACKED)
-                color = trace_dda_tex<false, TEX_PACKED>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err) * ec;
+                color = trace_dda_tex<false, TEX_PACKED, DDA_AHEAD_BATCH>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err) * ec;
             else
-                color = trace_dda_tex<false, TEX_RAW>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err) * ec;
+                color = trace_dda_tex<false, TEX_RAW, DDA_AHEAD_BATCH>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err) * ec;
         } else if constexpr (SPEC == XN_BATCH_ESVO_SHALLOW) {
             NodeStack<0> nodes{stk->a, stk->stride};
             V3 ro = f.translation + vs(1.0f);
@@ -2033,8 +2054,7 @@ __device__ __forceinline__ uint32_t render_job_pixel_spec(const BatchJob& J, uin
     }
 }
 
-// The texture-DDA forms are held to 32 registers (two blocks of 1024 per SM):
-// DDA hides texture latency with resident warps.
+// The texture-DDA forms are held to 32 registers (two blocks of 1024 per SM).
 constexpr int batch_min_blocks(int spec) {
     return spec == XN_BATCH_DDA_TEX_NORM || spec == XN_BATCH_DDA_TEX_RAW ? 2 : 1;
 }
