@@ -67,6 +67,7 @@ struct Levels {  // a BrickBuild as the kernels take it
     int L, Lb;
     uint32_t chan_diff;
     int sequential;
+    int equality;  // BrickBuild::equality
     double stddev;
     LevelGeom geo[MAX_LEVELS];
     uint64_t off[MAX_LEVELS + 1];
@@ -86,6 +87,7 @@ Levels levels_of(const BrickBuild& b) {
     a.Lb = b.Lb;
     a.chan_diff = b.chan_diff;
     a.sequential = b.sequential;
+    a.equality = b.equality;
     a.stddev = b.stddev;
     std::memcpy(a.geo, b.geo, sizeof a.geo);
     std::memcpy(a.off, b.off, sizeof a.off);
@@ -379,6 +381,40 @@ __device__ __forceinline__ void scan_octant(const Levels& a, const uint4 q[4], c
     }
 }
 
+// scan_octant where a cell is a leaf exactly when its voxels are equal
+// (ChannelDiff with threshold 0) and no colour but a leaf's is wanted: an OR of
+// differences a level instead of sums, minima and maxima (about a third of the
+// instructions).  A cell of unequal voxels has minimum 0 and maximum ~0.
+__device__ __forceinline__ void scan_octant_equality(const uint4 q[4], uint32_t lane, OctantSums& os,
+                                                     unsigned long long& l1, uint32_t& l2, uint32_t& l3) {
+    const uint32_t v = q[0].x, v1 = q[0].z;  // the first voxels of the lane's two cells
+    uint32_t d0 = q[0].y ^ v, d1 = q[0].w ^ v1;
+#pragma unroll
+    for (int r = 1; r < 4; ++r) {
+        d0 |= (q[r].x ^ v) | (q[r].y ^ v);
+        d1 |= (q[r].z ^ v1) | (q[r].w ^ v1);
+    }
+    const uint32_t in0 = __ballot_sync(FULL, d0 != 0), in1 = __ballot_sync(FULL, d1 != 0);
+    // the four lanes of a group against the first of them
+    const uint32_t dg = d0 | d1 | (v1 ^ v) | (__shfl_sync(FULL, v, lane & ~3u) ^ v);
+    uint32_t gbits = __ballot_sync(FULL, dg != 0);
+    gbits |= gbits >> 1;
+    gbits = (gbits | (gbits >> 2)) & 0x11111111u;  // bit 4 g
+    gbits = (gbits | (gbits >> 3)) & 0x03030303u;
+    gbits = (gbits | (gbits >> 6)) & 0x000F000Fu;
+    gbits = (gbits | (gbits >> 12)) & 0xFFu;
+    const bool octant = gbits || __any_sync(FULL, __shfl_sync(FULL, v, 0) != v);
+    if (lane == 0) {
+        os.s[0] = os.s[1] = os.s[2] = os.s[3] = 0;
+        os.mn = octant ? 0u : v;
+        os.mx = octant ? ~0u : v;
+        os.q = 0;
+        l1 = nibbles_to_bytes(in0) | (nibbles_to_bytes(in1) << 4);
+        l2 = gbits;
+        l3 = octant;
+    }
+}
+
 // One block per brick: the record, and the brick's size, colour, flags and
 // statistics.
 template <int HEUR, bool VEC>
@@ -413,7 +449,9 @@ __global__ void __launch_bounds__(BT) brick_scan_kernel(const __grid_constant__ 
 #pragma unroll
     for (uint32_t h = 0; h < 2; ++h) {
         const uint32_t o = h * 4 + warp;
-        if (whole) scan_octant<HEUR, true>(a, q[h], pl, lane, X + h * 8, OY, OZ, s_oct[o], s_l1[o], s_l2[o], s_l3[o]);
+        if (HEUR == XN_HEUR_CHANNEL_DIFF && whole && a.equality)
+            scan_octant_equality(q[h], lane, s_oct[o], s_l1[o], s_l2[o], s_l3[o]);
+        else if (whole) scan_octant<HEUR, true>(a, q[h], pl, lane, X + h * 8, OY, OZ, s_oct[o], s_l1[o], s_l2[o], s_l3[o]);
         else scan_octant<HEUR, false>(a, q[h], pl, lane, X + h * 8, OY, OZ, s_oct[o], s_l1[o], s_l2[o], s_l3[o]);
     }
     __syncthreads();
@@ -421,7 +459,8 @@ __global__ void __launch_bounds__(BT) brick_scan_kernel(const __grid_constant__ 
     const uint32_t o = lane & 7u;  // lanes 8.. repeat lanes 0..7
     OctantSums os = s_oct[o];
     const uint32_t on = count_in(a.g, X + (o >> 2) * 8, Y + ((o >> 1) & 1u) * 8, Z + (o & 1u) * 8, 8);
-    const uint32_t ocol = on ? average4(os.s[0], os.s[1], os.s[2], os.s[3], on) : 0u;
+    const bool by_value = HEUR == XN_HEUR_CHANNEL_DIFF && a.equality;  // only leaves' colours: their one value
+    const uint32_t ocol = by_value ? (on ? os.mn : 0u) : on ? average4(os.s[0], os.s[1], os.s[2], os.s[3], on) : 0u;
     Part p{};
     p.mn02 = os.mn & 0x00FF00FFu;
     p.mn13 = (os.mn >> 8) & 0x00FF00FFu;
@@ -463,7 +502,7 @@ __global__ void __launch_bounds__(BT) brick_scan_kernel(const __grid_constant__ 
         const uint32_t deep = !internal ? 0u : any1 ? 4u : any2 ? 3u : l3bits ? 2u : 1u;
         rec.top = l3bits | (internal ? ROOT_BIT : 0u) | (deep << 16);
         const uint32_t n = count_in(a.g, X, Y, Z, 16);
-        a.color[cell] = average4(os.s[0], os.s[1], os.s[2], os.s[3], n);
+        a.color[cell] = by_value ? p.mn02 | (p.mn13 << 8) : average4(os.s[0], os.s[1], os.s[2], os.s[3], n);
         a.flags[cell] = (internal ? 0 : F_LEAF) | F_INSIDE;
         if (HEUR == XN_HEUR_CHANNEL_DIFF) {
             CDStats& st = static_cast<CDStats*>(a.stats)[cell];
@@ -545,6 +584,7 @@ __device__ void up_cell(const Levels& a, int d, uint64_t i) {
         // _mm_subs_epu8(max, min), then the largest channel (Grid.cpp:124,135)
         const uint32_t dif = __vsubus4(mx, mn);
         split = max(max(dif & 0xFFu, (dif >> 8) & 0xFFu), max((dif >> 16) & 0xFFu, dif >> 24)) > a.chan_diff;
+        if (a.equality) avg = mn;
     } else {
         SDStats& out = static_cast<SDStats*>(a.stats)[cell];
         unsigned __int128 E = (unsigned __int128)n * q;  // n * sum((x - mean)^2), exact

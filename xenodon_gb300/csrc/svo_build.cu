@@ -610,6 +610,7 @@ int build_bricks(Ctx* c, const GridDev& g, uint64_t side, int L, bool ropes, int
     b.chan_diff = (uint32_t)(uint8_t)threshold;
     b.stddev = threshold;
     b.sequential = heuristic == XN_HEUR_STD_DEV && getenv("XN_BUILD_STDDEV_SEQUENTIAL") != nullptr;
+    b.equality = layout && heuristic == XN_HEUR_CHANNEL_DIFF && b.chan_diff == 0;
     const uint64_t bytes = brick_plan(b, side, nullptr);
     if (b.off[b.Lb + 1] > 0x70000000ull) return fail(XN_ERR_ARG, "xn_build_svo: grid too large");
     unsigned char* base = nullptr;

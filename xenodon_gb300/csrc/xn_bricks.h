@@ -56,6 +56,7 @@ struct BrickBuild {
     int heuristic;
     uint32_t chan_diff;
     double stddev;
+    int equality;    // ChannelDiff with threshold 0, and only the leaves' colours are wanted (not BRICK_NODES)
     int sequential;  // StdDev: every decision through the reference's loop (a check mode)
     LevelGeom geo[MAX_LEVELS];     // depths 0 .. Lb
     uint64_t off[MAX_LEVELS + 1];  // first cell of each depth in the arrays below
