@@ -43,7 +43,6 @@ int fill_table(Ctx* c, const xn_job* jobs, int n, uint32_t tile_w, void* table, 
     BatchJob* out = reinterpret_cast<BatchJob*>(h + 1);
     const uint32_t tile_h = 32 / tile_w;
     unsigned long long tiles = 0;
-    bool shallow = true;
     for (int i = 0; i < n; ++i) {
         const xn_job& j = jobs[i];
         if (!j.volume || !j.d_rgba) return fail(XN_ERR_ARG, "batch: job %d has no volume or output", i);
@@ -60,13 +59,8 @@ int fill_table(Ctx* c, const xn_job* jobs, int n, uint32_t tile_w, void* table, 
         tiles += (unsigned long long)out[i].tiles_x * out[i].tiles_y;
         const int sp = batch_spec(out[i]);
         out[i].form = sp;
-        shallow &= out[i].shallow != 0;
         if (spec_out) *spec_out = i == 0 ? sp : (*spec_out == sp ? sp : XN_BATCH_ANY);
     }
-    // a batch of one form on shallow octrees alone: fewer rows of stack or path a
-    // thread (batch graphs, whose jobs are not known yet, keep the full ones)
-    if (spec_out && n > 0 && shallow && *spec_out == XN_BATCH_ESVO) *spec_out = XN_BATCH_ESVO_SHALLOW;
-    if (spec_out && n > 0 && shallow && *spec_out == XN_BATCH_NAIVE) *spec_out = XN_BATCH_NAIVE_SHALLOW;
     h->n_jobs = (uint32_t)n;
     h->pad = 0;
     h->total_tiles = tiles;

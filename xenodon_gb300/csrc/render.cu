@@ -1869,8 +1869,8 @@ int batch_spec(const BatchJob& j) {
                              : XN_BATCH_ANY;
     if (j.layout != XN_LAYOUT_COMPACT) return XN_BATCH_ANY;
     switch (j.traversal) {
-    case XN_TRAV_ESVO: return XN_BATCH_ESVO;
-    case XN_TRAV_SVO_NAIVE: return XN_BATCH_NAIVE;
+    case XN_TRAV_ESVO: return j.shallow ? XN_BATCH_ESVO_SHALLOW : XN_BATCH_ESVO;
+    case XN_TRAV_SVO_NAIVE: return j.shallow ? XN_BATCH_NAIVE_SHALLOW : XN_BATCH_NAIVE;
     case XN_TRAV_SVO_DF: return !j.depth_consistent ? XN_BATCH_ANY : j.df_steps ? XN_BATCH_DF_STEPS : XN_BATCH_DF;
     case XN_TRAV_SVO_ROPE: return XN_BATCH_ROPE;
     default: return XN_BATCH_ANY;
@@ -2005,6 +2005,8 @@ __device__ __forceinline__ uint32_t render_job_pixel_spec(const BatchJob& J, uin
         case XN_BATCH_NAIVE: return render_job_pixel_spec<XN_BATCH_NAIVE>(J, ix, iy, true, err, stk);
         case XN_BATCH_ROPE: return render_job_pixel_spec<XN_BATCH_ROPE>(J, ix, iy, true, err, stk);
         case XN_BATCH_DF_STEPS: return render_job_pixel_spec<XN_BATCH_DF_STEPS>(J, ix, iy, true, err, stk);
+        case XN_BATCH_ESVO_SHALLOW: return render_job_pixel_spec<XN_BATCH_ESVO_SHALLOW>(J, ix, iy, true, err, stk);
+        case XN_BATCH_NAIVE_SHALLOW: return render_job_pixel_spec<XN_BATCH_NAIVE_SHALLOW>(J, ix, iy, true, err, stk);
         default: return render_job_pixel(J, ix, iy, err, stk);
         }
     } else {
