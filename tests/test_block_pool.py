@@ -1,0 +1,151 @@
+"""The rules of a context's device memory (xn_pool.h) over a counting
+allocator, and the bytes a budget's context really holds on the device."""
+from __future__ import annotations
+
+import subprocess
+from pathlib import Path
+
+import numpy as np
+import pytest
+
+ROOT = Path(__file__).resolve().parents[1]
+
+_DRIVER = r"""
+#include <cstdio>
+#include <cstdlib>
+#include <random>
+#include <thread>
+#include "xn_pool.h"
+static std::mutex g_mu;
+static std::unordered_map<void*, uint64_t> g_live;
+static uint64_t g_held = 0, g_most = 0, g_capacity = ~0ull, g_calls = 0;
+static int fake_alloc(void** p, uint64_t n) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    ++g_calls;
+    if (n > g_capacity - g_held) return 2;
+    *p = std::malloc(1);
+    g_live[*p] = n;
+    g_held += n;
+    if (g_held > g_most) g_most = g_held;
+    return 0;
+}
+static void fake_release(void* p) {
+    std::lock_guard<std::mutex> lk(g_mu);
+    auto it = g_live.find(p);
+    if (it == g_live.end()) { std::puts("released twice"); std::exit(1); }
+    g_held -= it->second;
+    g_live.erase(it);
+    std::free(p);
+}
+#define CHECK(x) do { if (!(x)) { std::printf("line %d: %s\n", __LINE__, #x); std::exit(1); } } while (0)
+using xn::BlockPool;
+static void churn(BlockPool& pool, unsigned seed, int steps) {
+    std::mt19937 r(seed);
+    std::vector<std::pair<void*, uint64_t>> mine;
+    for (int i = 0; i < steps; ++i) {
+        if (mine.empty() || r() % 5 < 3) {
+            const uint64_t n = (r() % 3 ? (r() % 40 + 1) << 20 : r() % (200 << 10) + 1) + r() % 3;
+            void* p;
+            const int e = pool.alloc(&p, n);
+            CHECK(e == 0 ? p != nullptr : p == nullptr && (e == BlockPool::OVER_BUDGET || e == 2));
+            if (!e) mine.push_back({p, n});
+        } else {
+            const size_t k = r() % mine.size();
+            pool.free(mine[k].first, mine[k].second, r() % 4 != 0);
+            mine.erase(mine.begin() + k);
+        }
+    }
+    for (auto& b : mine) pool.free(b.first, b.second, true);
+}
+int main() {
+    const BlockPool::Api api{fake_alloc, fake_release, 2};
+    const uint64_t MB = 1 << 20;
+    {   // a budget bounds what is held at every moment, from several threads too
+        BlockPool pool(api);
+        pool.budget = 256 * MB;
+        pool.cap = 10000 * MB;
+        churn(pool, 1, 20000);
+        std::vector<std::thread> t;
+        for (unsigned s = 2; s < 6; ++s) t.emplace_back(churn, std::ref(pool), s, 5000);
+        for (auto& x : t) x.join();
+        CHECK(g_most <= 256 * MB && g_most > 200 * MB && pool.used == 0);
+        void* p;
+        CHECK(pool.alloc(&p, 256 * MB) == 0 && g_held == 256 * MB);  // all of it for one block
+        void* q;
+        CHECK(pool.alloc(&q, 1) == BlockPool::OVER_BUDGET && pool.used == 256 * MB);
+        pool.free(p, 256 * MB, true);
+        const uint64_t calls = g_calls;
+        CHECK(pool.alloc(&p, 256 * MB) == 0 && g_calls == calls);  // the kept block again
+        pool.free(p, 256 * MB, true);
+        CHECK(pool.reserve(200 * MB) && g_held == 0);  // memory that the caller allocates itself makes room too
+        CHECK(!pool.reserve(57 * MB) && pool.reserve(56 * MB));
+        pool.unreserve(256 * MB);
+    }
+    {   // without one: at most cap bytes are kept; of busy blocks none
+        BlockPool pool(api);
+        pool.cap = 100 * MB;
+        churn(pool, 7, 20000);
+        CHECK(g_held <= 100 * MB && g_held > 0 && pool.used == 0);
+        pool.trim(0);
+        CHECK(g_held == 0);
+        void* p;
+        CHECK(pool.alloc(&p, 50 * MB) == 0);
+        pool.free(p, 50 * MB, false);
+        CHECK(g_held == 0);
+        void* q;
+        CHECK(pool.alloc(&p, 50 * MB) == 0);
+        pool.free(p, 50 * MB, true);
+        CHECK(pool.alloc(&q, 49 * MB) == 0 && q == p);  // a block of about the size
+        pool.free(q, 49 * MB, true);
+        // short of memory: the kept blocks are given back, then the exact size is tried
+        g_capacity = 65 * MB + 1;
+        CHECK(pool.alloc(&p, 65 * MB + 1) == 0 && g_held == g_capacity);
+        CHECK(pool.alloc(&q, 1) == 2 && q == nullptr && pool.used == 65 * MB + 1);
+        pool.free(p, 65 * MB + 1, true);
+        pool.trim(0);
+        CHECK(g_held == 0 && pool.used == 0);
+    }
+    std::puts("ok");
+}
+"""
+
+
+def test_pool_rules(tmp_path):
+    src, exe = tmp_path / "pool.cpp", tmp_path / "pool"
+    src.write_text(_DRIVER)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", str(ROOT / "xenodon_gb300" / "csrc"), str(src), "-o", str(exe),
+                    "-lpthread"], check=True)
+    r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+@pytest.mark.gpu
+def test_budget_bounds_the_memory_held(built_library, monkeypatch):
+    """Volumes just above a rounding step, then a larger one, while freed
+    blocks are kept.  The device hands memory out in steps of 2 MB."""
+    import torch
+    import xenodon_gb300 as xg
+    monkeypatch.setenv("XN_GRID_LAYOUT", "linear")
+    mb = 1 << 20
+    g = np.zeros((1, 4097, 4096, 4), np.uint8)  # 64 MB and 16 KB
+    n = 12
+    with xg.Context(0) as warm:
+        warm.upload_grid(g).release()
+    with xg.Context(0, hbm_budget=n * g.nbytes + 4) as c:  # and the context's error word
+        free0 = torch.cuda.mem_get_info()[0]
+
+        def held():
+            return free0 - torch.cuda.mem_get_info()[0]
+
+        for _ in range(2):
+            vols = [c.upload_grid(g) for _ in range(n)]
+            assert held() <= n * (g.nbytes + 2 * mb)
+            for v in vols:
+                v.release()
+            assert held() <= n * (g.nbytes + 2 * mb)
+        big = c.upload_grid(np.zeros((2, 8192, 4096, 4), np.uint8))
+        assert held() <= n * (g.nbytes + 2 * mb)
+        with pytest.raises(xg.XenodonError) as e:
+            [c.upload_grid(g) for _ in range(n)]
+        assert e.value.code == xg.XN_ERR_BUDGET
+        big.release()

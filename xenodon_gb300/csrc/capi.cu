@@ -6,7 +6,6 @@
 // with one CUDA device context per xn_ctx.  No C++ exception crosses the ABI:
 // every entry point catches, records a message for xn_last_error() and
 // returns a status.
-#include <algorithm>
 #include <atomic>
 #include <cstdarg>
 #include <cstdio>
@@ -45,93 +44,28 @@ int cuda_fail(cudaError_t e, const char* what) {
                 cudaGetErrorString(e));
 }
 
-// Sizes are rounded up to a 16th of their power of two, so that the next
-// octree of about the same size finds the last one's block.
-static uint64_t block_size(uint64_t bytes) {
-    uint64_t unit = 512;
-    while (unit * 32 <= bytes) unit <<= 1;
-    return (bytes + unit - 1) / unit * unit;
+static int pool_alloc(void** p, uint64_t bytes) {
+    const cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return (int)e;
 }
+static void pool_release(void* p) { cudaFree(p); }
 
-constexpr uint64_t POOL_SMALLEST = 64 << 10;
-
-void Ctx::trim_pool(uint64_t keep) {
-    std::lock_guard<std::mutex> lk(pool_mu);
-    size_t n = 0;
-    while (pool_bytes > keep && n < pool.size()) {
-        cudaFree(pool[n].p);
-        pool_bytes -= pool[n++].bytes;
-    }
-    pool.erase(pool.begin(), pool.begin() + (std::ptrdiff_t)n);
-}
+Ctx::Ctx() : pool(BlockPool::Api{pool_alloc, pool_release, (int)cudaErrorMemoryAllocation}) {}
 
 int Ctx::device_alloc(void** p, uint64_t bytes, const char* what) {
     *p = nullptr;
     if (bytes == 0) return XN_OK;
-    uint64_t cur = used.load();
-    if (budget && cur + bytes > budget)
+    const int e = pool.alloc(p, bytes);
+    if (e == BlockPool::OVER_BUDGET)
         return fail(XN_ERR_BUDGET, "%s: %llu bytes exceed the HBM budget (%llu of %llu bytes in use)", what,
-                    (unsigned long long)bytes, (unsigned long long)cur, (unsigned long long)budget);
-    uint64_t size = block_size(bytes);
-    {
-        std::lock_guard<std::mutex> lk(pool_mu);
-        size_t best = pool.size();
-        for (size_t i = 0; i < pool.size(); ++i)
-            if (pool[i].bytes >= size && pool[i].bytes <= size + size / 8 &&
-                (best == pool.size() || pool[i].bytes < pool[best].bytes))
-                best = i;
-        if (best < pool.size()) {
-            *p = pool[best].p;
-            pool_bytes -= pool[best].bytes;
-            sizes[*p] = pool[best].bytes;
-            pool.erase(pool.begin() + (std::ptrdiff_t)best);
-        }
-    }
-    if (!*p) {
-        cudaError_t e = cudaMalloc(p, size);
-        if (e == cudaErrorMemoryAllocation) {  // without the pool, and without the rounding
-            cudaGetLastError();
-            trim_pool(0);
-            size = bytes;
-            e = cudaMalloc(p, size);
-        }
-        if (e != cudaSuccess) {
-            *p = nullptr;
-            return cuda_fail(e, what);
-        }
-        std::lock_guard<std::mutex> lk(pool_mu);
-        sizes[*p] = size;
-    }
-    used += bytes;
-    if (budget) {
-        const uint64_t now = used.load();
-        trim_pool(now < budget ? budget - now : 0);
-    }
-    return XN_OK;
+                    (unsigned long long)bytes, (unsigned long long)pool.used.load(), (unsigned long long)pool.budget);
+    return e ? cuda_fail((cudaError_t)e, what) : XN_OK;
 }
 
 void Ctx::device_free(void* p, uint64_t bytes) {
     if (!p) return;
-    used -= bytes;
-    uint64_t size = 0;
-    {
-        std::lock_guard<std::mutex> lk(pool_mu);
-        auto it = sizes.find(p);
-        if (it != sizes.end()) {
-            size = it->second;
-            sizes.erase(it);
-        }
-    }
-    const uint64_t now = used.load();
-    const uint64_t room = !budget ? pool_cap : now < budget ? std::min(pool_cap, budget - now) : 0;
-    if (size < POOL_SMALLEST || size > room || cudaDeviceSynchronize() != cudaSuccess) {
-        cudaFree(p);
-        return;
-    }
-    trim_pool(room - size);
-    std::lock_guard<std::mutex> lk(pool_mu);
-    pool.push_back({p, size});
-    pool_bytes += size;
+    pool.free(p, bytes, bytes >= BlockPool::SMALLEST && cudaDeviceSynchronize() == cudaSuccess);
 }
 
 int Ctx::ensure_buffer(DeviceBuffer& b, uint64_t bytes, const char* what) {
@@ -177,7 +111,7 @@ XN_API int xn_create(int device, uint64_t hbm_budget_bytes, xn_ctx** out) {
     Ctx* c = new (std::nothrow) Ctx();
     if (!c) return fail(XN_ERR_NOMEM, "xn_create: out of host memory");
     c->device = device;
-    c->budget = hbm_budget_bytes;
+    c->pool.budget = hbm_budget_bytes;
     int r = c->activate();
     if (r) { delete c; return r; }
     if ((e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking)) != cudaSuccess ||
@@ -192,7 +126,7 @@ XN_API int xn_create(int device, uint64_t hbm_budget_bytes, xn_ctx** out) {
     cudaMemsetAsync(c->d_err, 0, sizeof(uint32_t), c->stream);
     cudaStreamSynchronize(c->stream);
     size_t free_bytes = 0, total_bytes = 0;
-    if (cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess) c->pool_cap = total_bytes / 32;
+    if (cudaMemGetInfo(&free_bytes, &total_bytes) == cudaSuccess) c->pool.cap = total_bytes / 32;
     *out = reinterpret_cast<xn_ctx*>(c);
     return XN_OK;
 }
@@ -205,7 +139,7 @@ XN_API int xn_destroy(xn_ctx* h) {
     c->device_free(c->out_rgba.ptr, c->out_rgba.bytes);
     c->device_free(c->out_emission.ptr, c->out_emission.bytes);
     c->device_free(c->d_err, sizeof(uint32_t));
-    c->trim_pool(0);
+    c->pool.trim(0);
     c->release_extra();
     if (c->ev0) cudaEventDestroy(c->ev0);
     if (c->ev1) cudaEventDestroy(c->ev1);
@@ -217,8 +151,8 @@ XN_API int xn_destroy(xn_ctx* h) {
 XN_API int xn_ctx_memory(const xn_ctx* h, uint64_t* used_bytes, uint64_t* budget_bytes) {
     if (!h) return fail(XN_ERR_ARG, "xn_ctx_memory: ctx is NULL");
     const Ctx* c = reinterpret_cast<const Ctx*>(h);
-    if (used_bytes) *used_bytes = c->used.load();
-    if (budget_bytes) *budget_bytes = c->budget;
+    if (used_bytes) *used_bytes = c->pool.used.load();
+    if (budget_bytes) *budget_bytes = c->pool.budget;
     return XN_OK;
 }
 
@@ -361,7 +295,7 @@ int upload_grid(xn_ctx* h, const uint8_t* rgba, bool from_device, uint32_t dx, u
         const char* rd = std::getenv("XN_TEX_READ");
         const bool packed = rd && std::strcmp(rd, "packed") == 0;
         const bool norm = !packed && !(rd && std::strcmp(rd, "raw") == 0) && texture_unorm_exact(c) == 1;
-        if (c->budget && c->used.load() + bytes > c->budget) {
+        if (!c->pool.reserve(bytes)) {
             delete v;
             return fail(XN_ERR_BUDGET, "xn_volume_upload_grid: %llu bytes exceed the HBM budget",
                         (unsigned long long)bytes);
@@ -370,19 +304,15 @@ int upload_grid(xn_ctx* h, const uint8_t* rgba, bool from_device, uint32_t dx, u
         e = cudaMalloc3DArray(&v->array, &d, make_cudaExtent(dx, dy, dz));
         if (e == cudaErrorMemoryAllocation) {
             cudaGetLastError();
-            c->trim_pool(0);
+            c->pool.trim(0);
             e = cudaMalloc3DArray(&v->array, &d, make_cudaExtent(dx, dy, dz));
         }
         if (e != cudaSuccess) {
+            c->pool.unreserve(bytes);
             delete v;
             return cuda_fail(e, "xn_volume_upload_grid: array");
         }
         v->array_bytes = bytes;
-        c->used += bytes;
-        if (c->budget) {
-            const uint64_t now = c->used.load();
-            c->trim_pool(now < c->budget ? c->budget - now : 0);
-        }
         cudaMemcpy3DParms p = {};
         p.srcPtr = make_cudaPitchedPtr(const_cast<uint8_t*>(rgba), (size_t)dx * 4, dx, dy);
         p.dstArray = v->array;
@@ -400,7 +330,7 @@ int upload_grid(xn_ctx* h, const uint8_t* rgba, bool from_device, uint32_t dx, u
             if ((r = c->device_alloc(&v->data, bytes, "xn_volume_upload_grid: linear copy"))) {
                 cudaDestroyTextureObject(v->tex);
                 cudaFreeArray(v->array);
-                c->used -= bytes;
+                c->pool.unreserve(bytes);
                 delete v;
                 return r;
             }
@@ -415,7 +345,7 @@ int upload_grid(xn_ctx* h, const uint8_t* rgba, bool from_device, uint32_t dx, u
         }
         if (e != cudaSuccess) {
             cudaFreeArray(v->array);
-            c->used -= bytes;
+            c->pool.unreserve(bytes);
             delete v;
             return cuda_fail(e, "xn_volume_upload_grid: texture");
         }
@@ -542,7 +472,7 @@ XN_API int xn_volume_release(xn_volume* h) {
     if (v->tex) cudaDestroyTextureObject(v->tex);
     if (v->array) {
         cudaFreeArray(v->array);
-        c->used -= v->array_bytes;
+        c->pool.unreserve(v->array_bytes);
     }
     delete v;
     return XN_OK;

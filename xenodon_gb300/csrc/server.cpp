@@ -120,7 +120,7 @@ struct Pool {
         cudaError_t e = device ? cudaMalloc(&p, r) : cudaHostAlloc(&p, r, cudaHostAllocDefault);
         if (device && e == cudaErrorMemoryAllocation) {  // the context's freed blocks may be in the way
             cudaGetLastError();
-            ctx->trim_pool(0);
+            ctx->pool.trim(0);
             e = cudaMalloc(&p, r);
         }
         if (e != cudaSuccess) return nullptr;

@@ -1,15 +1,13 @@
 // Host-side state behind the opaque xn_ctx / xn_volume handles.
 #pragma once
 
-#include <atomic>
 #include <cstdint>
 #include <mutex>
-#include <unordered_map>
-#include <vector>
 
 #include <cuda_runtime.h>
 
 #include "../../include/xenodon.h"
+#include "xn_pool.h"
 
 namespace xn {
 
@@ -22,8 +20,6 @@ struct DeviceBuffer {
 // context is checked against.
 struct Ctx {
     int device = 0;
-    uint64_t budget = 0;  // 0 = no cap
-    std::atomic<uint64_t> used{0};
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     uint32_t* d_err = nullptr;  // ray error bits
@@ -37,23 +33,9 @@ struct Ctx {
     xn_batch_config tuned[32] = {};
     int tuned_valid[32] = {};
     std::mutex mu;
-    // Freed device memory kept for the next allocations: a 4.3 GB octree's
-    // cudaMalloc and cudaFree take 0.6 and 1.8 ms, more than half of its build's
-    // kernels.  At most pool_cap bytes (a 32nd of the device's memory), the
-    // oldest given back first; all of it when an allocation fails or the
-    // context goes, and what a budget leaves no room for at once.  A block
-    // enters the pool after a device synchronisation, as cudaFree implies one,
-    // so no stream still uses it.
-    struct Block {
-        void* p;
-        uint64_t bytes;
-    };
-    std::mutex pool_mu;
-    std::vector<Block> pool;                    // oldest first
-    std::unordered_map<void*, uint64_t> sizes;  // of the blocks in use
-    uint64_t pool_bytes = 0, pool_cap = 0;
+    BlockPool pool;  // every device allocation, its budget, and freed blocks kept
+    Ctx();
 
-    void trim_pool(uint64_t keep);  // gives blocks back until at most `keep` bytes are pooled
     int sm_count();
 
     int activate();
