@@ -123,6 +123,11 @@ bool generic_forced() {
 
 int render_batch_one(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& cfg, cudaStream_t s);
 
+void launched(Ctx* c, const xn_job* jobs, int n, cudaStream_t s) {
+    if (c->track_launch(s)) return;
+    for (int i = 0; i < n; ++i) reinterpret_cast<const Volume*>(jobs[i].volume)->untracked = true;
+}
+
 // The plain form: every job through the single-frame kernels, one launch
 // each, in order on the stream (the reference's one dispatch per frame,
 // src/render/Renderer.cpp:74-89, with its launch shape and register budget).
@@ -145,7 +150,7 @@ int render_plain(Ctx* c, const xn_job* jobs, int n, cudaStream_t s) {
 // A batch whose jobs need different kernel forms runs as one launch per form
 // (each specialised, each over its own jobs, in the stream's order); with
 // XN_BATCH_GENERIC=1 the generic form takes the whole batch in one launch.
-int render_batch_locked(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& cfg, cudaStream_t s) {
+int render_batch_forms(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& cfg, cudaStream_t s) {
     if (cfg.tile_width == XN_BATCH_PLAIN) return render_plain(c, jobs, n, s);
     if (!generic_forced()) {
         std::vector<int> forms;
@@ -165,6 +170,14 @@ int render_batch_locked(Ctx* c, const xn_job* jobs, int n, const xn_batch_config
         }
     }
     return render_batch_one(c, jobs, n, cfg, s);
+}
+
+int render_batch_locked(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& cfg, cudaStream_t s) {
+    for (int i = 0; i < n; ++i)
+        if (!jobs[i].volume) return fail(XN_ERR_ARG, "batch: job %d has no volume or output", i);
+    const int r = render_batch_forms(c, jobs, n, cfg, s);
+    launched(c, jobs, n, s);  // also after an error: a part may have been launched
+    return r;
 }
 
 int render_batch_one(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& cfg, cudaStream_t s) {
@@ -438,6 +451,7 @@ XN_API int xn_batch_graph_launch(xn_batch_graph* g, const xn_job* jobs, int n) {
         return r;
     }
     cudaError_t e = cudaGraphLaunch(sl.exec, g->stream);
+    launched(c, jobs, n, g->stream);
     if (e == cudaSuccess) e = cudaEventRecord(sl.done, g->stream);
     if (e != cudaSuccess) return cuda_fail(e, "xn_batch_graph_launch");
     sl.pending = true;

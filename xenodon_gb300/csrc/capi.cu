@@ -63,9 +63,65 @@ int Ctx::device_alloc(void** p, uint64_t bytes, const char* what) {
     return e ? cuda_fail((cudaError_t)e, what) : XN_OK;
 }
 
-void Ctx::device_free(void* p, uint64_t bytes) {
+void Ctx::device_free(void* p, uint64_t bytes, bool tracked) {
     if (!p) return;
-    pool.free(p, bytes, bytes >= BlockPool::SMALLEST && cudaDeviceSynchronize() == cudaSuccess);
+    pool.free(p, bytes, tracked && bytes >= BlockPool::SMALLEST && wait_launches());
+}
+
+// 0.3 us of host time (a launch with it 3.4 us, without 3.1).
+bool Ctx::track_launch(cudaStream_t s) {
+    if (s == stream) return true;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    unsigned long long id = 0;
+    cudaError_t e = cudaStreamIsCapturing(s, &capture);
+    if (e == cudaSuccess && capture != cudaStreamCaptureStatusNone) return false;
+    if (e == cudaSuccess) e = cudaStreamGetId(s, &id);
+    std::lock_guard<std::mutex> lk(launch_mu);
+    Launch* l = nullptr;
+    for (Launch& k : launches)
+        if (k.stream_id == id) l = &k;
+    if (e == cudaSuccess && !l && launches.size() < MOST_LAUNCHES) {
+        cudaEvent_t ev = nullptr;
+        if (!spare_events.empty()) {
+            ev = spare_events.back();
+            spare_events.pop_back();
+        } else {
+            e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+        }
+        if (e == cudaSuccess) {
+            launches.push_back({id, ev, 0});
+            l = &launches.back();
+        }
+    }
+    if (e == cudaSuccess && l) {
+        l->turn = ++launch_turn;
+        e = cudaEventRecord(l->done, s);
+    }
+    if (e != cudaSuccess) cudaGetLastError();
+    return e == cudaSuccess && l;
+}
+
+bool Ctx::wait_launches() {
+    cudaError_t e = cudaStreamSynchronize(stream);
+    std::vector<Launch> wait;
+    {
+        std::lock_guard<std::mutex> lk(launch_mu);
+        wait = launches;
+    }
+    for (size_t i = 0; i < wait.size() && e == cudaSuccess; ++i) e = cudaEventSynchronize(wait[i].done);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    std::lock_guard<std::mutex> lk(launch_mu);
+    for (const Launch& w : wait)
+        for (size_t i = 0; i < launches.size(); ++i)
+            if (launches[i].stream_id == w.stream_id && launches[i].turn == w.turn) {
+                spare_events.push_back(w.done);
+                launches.erase(launches.begin() + (std::ptrdiff_t)i);
+                break;
+            }
+    return true;
 }
 
 int Ctx::ensure_buffer(DeviceBuffer& b, uint64_t bytes, const char* what) {
@@ -84,6 +140,8 @@ void Ctx::release_extra() {
         cudaEventDestroy(batch_copied);
     }
     if (batch_host) cudaFreeHost(batch_host);
+    for (Launch& l : launches) cudaEventDestroy(l.done);
+    for (cudaEvent_t ev : spare_events) cudaEventDestroy(ev);
 }
 
 int Ctx::activate() {
@@ -467,7 +525,7 @@ XN_API int xn_volume_release(xn_volume* h) {
     std::lock_guard<std::mutex> lk(c->mu);
     c->activate();
     cudaStreamSynchronize(c->stream);
-    c->device_free(v->data, v->bytes);
+    c->device_free(v->data, v->bytes, !v->untracked);
     v->release_layout();
     if (v->tex) cudaDestroyTextureObject(v->tex);
     if (v->array) {
@@ -641,6 +699,7 @@ XN_API int xn_render_device(xn_ctx* h, const xn_volume* vh, int traversal, const
     r = c->activate();
     if (r) return r;
     cudaError_t e = launch_render(L, static_cast<cudaStream_t>(stream));
+    v->launched(static_cast<cudaStream_t>(stream));
     return e == cudaSuccess ? XN_OK : cuda_fail(e, "xn_render_device: launch");
 }
 

@@ -139,6 +139,7 @@ XN_API int xn_output_destroy(xn_output* oh) {
     std::lock_guard<std::mutex> lk(c->mu);
     c->activate();
     if (o->pending) cudaEventSynchronize(o->done);
+    cudaStreamSynchronize(o->copy);
     c->device_free(o->d_rgba, o->max_pixels * 4);
     c->device_free(o->d_err, 4);
     cudaFreeHost(o->h_rgba);

@@ -1,8 +1,10 @@
 // Host-side state behind the opaque xn_ctx / xn_volume handles.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <mutex>
+#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -36,11 +38,31 @@ struct Ctx {
     BlockPool pool;  // every device allocation, its budget, and freed blocks kept
     Ctx();
 
+    // Launches on streams that are not the context's, so that freed memory can
+    // wait for them: the last one of each stream (by the stream's id; handles
+    // are used again).  A device synchronisation would do as well, but it
+    // invalidates every stream capture that is under way in the process.  (The
+    // render server's folding kernel is not among them: its volumes are released
+    // when their requests are done, and then it reads them no more.)
+    struct Launch {
+        unsigned long long stream_id;
+        cudaEvent_t done;
+        uint64_t turn;  // changes with each launch
+    };
+    static constexpr size_t MOST_LAUNCHES = 64;
+    std::mutex launch_mu;
+    std::vector<Launch> launches;
+    std::vector<cudaEvent_t> spare_events;
+    uint64_t launch_turn = 0;
+    bool track_launch(cudaStream_t s);  // false: the end of this launch is not known
+    bool wait_launches();               // waits for the context's stream and all tracked launches; false: not known
+
     int sm_count();
 
     int activate();
     int device_alloc(void** p, uint64_t bytes, const char* what);
-    void device_free(void* p, uint64_t bytes);
+    // tracked: every launch that uses the block is on the context's stream or tracked
+    void device_free(void* p, uint64_t bytes, bool tracked = true);
     int ensure_buffer(DeviceBuffer& b, uint64_t bytes, const char* what);
     void release_extra();
 };
@@ -75,12 +97,20 @@ struct Volume {
         return (inner ? n_inner * 32 : 0) + (rinner ? n_inner * 32 : 0) + (inner_depth ? n_inner * 4 : 0) +
                (leaves ? n_leaves * 32 : 0);
     }
+    // Set by a launch whose end is not known (one that is being captured: its
+    // graph may be replayed at any time): the memory goes back to the device,
+    // whose own free waits for it.
+    mutable std::atomic<bool> untracked{false};
+    void launched(cudaStream_t s) const {
+        if (!ctx->track_launch(s)) untracked = true;
+    }
+
     void release_layout() {
         if (!ctx) return;
-        ctx->device_free(inner, n_inner * 32);
-        ctx->device_free(rinner, n_inner * 32);
-        ctx->device_free(inner_depth, n_inner * 4);
-        ctx->device_free(leaves, n_leaves * 32);
+        ctx->device_free(inner, n_inner * 32, !untracked);
+        ctx->device_free(rinner, n_inner * 32, !untracked);
+        ctx->device_free(inner_depth, n_inner * 4, !untracked);
+        ctx->device_free(leaves, n_leaves * 32, !untracked);
         inner = rinner = inner_depth = leaves = nullptr;
     }
 };
