@@ -102,7 +102,11 @@ int main() {
         CHECK(pool.alloc(&p, 65 * MB + 1) == 0 && g_held == g_capacity);
         CHECK(pool.alloc(&q, 1) == 2 && q == nullptr && pool.used == 65 * MB + 1);
         pool.free(p, 65 * MB + 1, true);
-        pool.trim(0);
+        // and for an allocation that does not go through the pool
+        CHECK(g_held == 65 * MB + 1);
+        CHECK(pool.with_room([&] { return fake_alloc(&q, 60 * MB); }) == 0 && g_held == 60 * MB);
+        CHECK(pool.with_room([&] { return fake_alloc(&p, 60 * MB); }) == 2);
+        fake_release(q);
         CHECK(g_held == 0 && pool.used == 0);
     }
     std::puts("ok");
@@ -117,6 +121,20 @@ def test_pool_rules(tmp_path):
                     "-lpthread"], check=True)
     r = subprocess.run([str(exe)], capture_output=True, text=True, timeout=120)
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+def test_every_device_allocation_has_the_kept_blocks_to_fall_back_on():
+    """A failed allocation is tried again without the kept blocks, wherever the
+    library asks the device for memory."""
+    import re
+    bad = []
+    for f in sorted((ROOT / "xenodon_gb300" / "csrc").iterdir()):
+        for n, line in enumerate(f.read_text().splitlines(), 1):
+            code = line.split("//")[0]
+            if re.search(r"\bcudaMalloc(Async|3DArray|Array|3D|Pitch|Managed)?\(|cudaGraphInstantiate\(", code) and \
+                    "with_room(" not in code and "BlockPool::alloc tries again" not in line:
+                bad.append(f"{f.name}:{n}: {line.strip()}")
+    assert not bad
 
 
 @pytest.mark.gpu

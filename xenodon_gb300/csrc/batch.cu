@@ -193,7 +193,7 @@ int render_batch_one(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& c
     if (generic_forced()) spec = XN_BATCH_ANY;
     const uint64_t queue_off = (bytes + 255) & ~255ull;
     void* d = nullptr;
-    e = cudaMallocAsync(&d, queue_off + 256, s);
+    e = c->with_room([&] { return cudaMallocAsync(&d, queue_off + 256, s); });
     if (e != cudaSuccess) return cuda_fail(e, "xn_render_batch: job table");
     unsigned long long* queue = reinterpret_cast<unsigned long long*>(static_cast<char*>(d) + queue_off);
     e = cudaMemcpyAsync(d, c->batch_host, bytes, cudaMemcpyHostToDevice, s);
@@ -413,7 +413,7 @@ XN_API int xn_batch_graph_create(xn_ctx* h, int capacity, const xn_batch_config*
                          g->cfg.block_threads, blocks, g->cfg.chunk, g->split ? f : XN_BATCH_ANY, cap);
         cudaGraph_t graph = nullptr;
         e = cudaStreamEndCapture(cap, &graph);
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&sl.exec, graph, 0);
+        if (e == cudaSuccess) e = c->with_room([&] { return cudaGraphInstantiate(&sl.exec, graph, 0); });
         if (graph) cudaGraphDestroy(graph);
     }
     if (cap) cudaStreamDestroy(cap);

@@ -45,7 +45,7 @@ int cuda_fail(cudaError_t e, const char* what) {
 }
 
 static int pool_alloc(void** p, uint64_t bytes) {
-    const cudaError_t e = cudaMalloc(p, bytes);
+    const cudaError_t e = cudaMalloc(p, bytes);  // BlockPool::alloc tries again
     if (e != cudaSuccess) cudaGetLastError();
     return (int)e;
 }
@@ -283,7 +283,7 @@ int texture_unorm_exact(Ctx* c) {
     c->tex_norm_exact = 0;
     cudaChannelFormatDesc d = cudaCreateChannelDesc<uchar4>();
     cudaArray_t a = nullptr;
-    if (cudaMalloc3DArray(&a, &d, make_cudaExtent(256, 1, 1)) != cudaSuccess) return 0;
+    if (c->with_room([&] { return cudaMalloc3DArray(&a, &d, make_cudaExtent(256, 1, 1)); }) != cudaSuccess) return 0;
     uchar4 h[256];
     for (int i = 0; i < 256; ++i) h[i] = make_uchar4(i, 255 - i, i, 255 - i);
     cudaMemcpy3DParms p = {};
@@ -295,7 +295,7 @@ int texture_unorm_exact(Ctx* c) {
     cudaTextureObject_t t = 0;
     unsigned hb = 1;
     if (cudaMemcpy3DAsync(&p, c->stream) == cudaSuccess && (t = make_texture(a, true)) != 0 &&
-        cudaMallocAsync(reinterpret_cast<void**>(&bad), 4, c->stream) == cudaSuccess &&
+        c->with_room([&] { return cudaMallocAsync(reinterpret_cast<void**>(&bad), 4, c->stream); }) == cudaSuccess &&
         cudaMemsetAsync(bad, 0, 4, c->stream) == cudaSuccess) {
         tex_unorm_check_kernel<<<1, 256, 0, c->stream>>>(t, bad);
         if (cudaMemcpyAsync(&hb, bad, 4, cudaMemcpyDeviceToHost, c->stream) != cudaSuccess) hb = 1;
@@ -359,12 +359,7 @@ int upload_grid(xn_ctx* h, const uint8_t* rgba, bool from_device, uint32_t dx, u
                         (unsigned long long)bytes);
         }
         cudaChannelFormatDesc d = packed ? cudaCreateChannelDesc<unsigned int>() : cudaCreateChannelDesc<uchar4>();
-        e = cudaMalloc3DArray(&v->array, &d, make_cudaExtent(dx, dy, dz));
-        if (e == cudaErrorMemoryAllocation) {
-            cudaGetLastError();
-            c->pool.trim(0);
-            e = cudaMalloc3DArray(&v->array, &d, make_cudaExtent(dx, dy, dz));
-        }
+        e = c->with_room([&] { return cudaMalloc3DArray(&v->array, &d, make_cudaExtent(dx, dy, dz)); });
         if (e != cudaSuccess) {
             c->pool.unreserve(bytes);
             delete v;
@@ -490,7 +485,8 @@ XN_API int xn_volume_upload_svo(xn_ctx* h, const uint32_t* nodes, uint64_t n_nod
     if (r) { delete v; return r; }
     cudaError_t e = cudaMemcpyAsync(v->data, nodes, v->bytes, cudaMemcpyHostToDevice, c->stream);
     uint32_t* flags = nullptr;  // [0] = bad index, [1] = has ropes
-    if (e == cudaSuccess) e = cudaMallocAsync(reinterpret_cast<void**>(&flags), 8, c->stream);
+    if (e == cudaSuccess)
+        e = c->with_room([&] { return cudaMallocAsync(reinterpret_cast<void**>(&flags), 8, c->stream); });
     if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, 8, c->stream);
     if (e == cudaSuccess) {
         validate_nodes_kernel<<<1024, 256, 0, c->stream>>>(static_cast<const uint32_t*>(v->data), n_nodes, flags);

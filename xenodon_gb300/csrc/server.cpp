@@ -117,12 +117,8 @@ struct Pool {
             return p;
         }
         void* p = nullptr;
-        cudaError_t e = device ? cudaMalloc(&p, r) : cudaHostAlloc(&p, r, cudaHostAllocDefault);
-        if (device && e == cudaErrorMemoryAllocation) {  // the context's freed blocks may be in the way
-            cudaGetLastError();
-            ctx->pool.trim(0);
-            e = cudaMalloc(&p, r);
-        }
+        const cudaError_t e = device ? ctx->with_room([&] { return cudaMalloc(&p, r); })
+                                     : cudaHostAlloc(&p, r, cudaHostAllocDefault);
         if (e != cudaSuccess) return nullptr;
         all.emplace_back(p, r);
         *got = r;
@@ -681,11 +677,13 @@ XN_API int xn_server_create(xn_ctx* ctx, const xn_server_config* cfg, xn_server*
         if (ok) s->large_streams.push_back(st);
     }
     const uint64_t cap = (uint64_t)s->cfg.max_batch_jobs;
+    auto device = [&](auto** p, uint64_t bytes) {
+        return s->c->with_room([&] { return cudaMalloc(reinterpret_cast<void**>(p), bytes); }) == cudaSuccess;
+    };
     for (auto& r : s->rings) {
         if (!ok) break;
-        ok = cudaMalloc(reinterpret_cast<void**>(&r.d_ctl), sizeof(xn::FoldCtl)) == cudaSuccess &&
-             cudaMalloc(reinterpret_cast<void**>(&r.d_ring), cap * sizeof(xn::BatchJob)) == cudaSuccess &&
-             cudaMalloc(reinterpret_cast<void**>(&r.d_done_tiles), cap * 4) == cudaSuccess &&
+        ok = device(&r.d_ctl, sizeof(xn::FoldCtl)) && device(&r.d_ring, cap * sizeof(xn::BatchJob)) &&
+             device(&r.d_done_tiles, cap * 4) &&
              cudaStreamCreateWithPriority(&r.stream, cudaStreamNonBlocking, hi) == cudaSuccess &&
              cudaHostAlloc(reinterpret_cast<void**>(&r.h_done), (cap + 1) * 4, cudaHostAllocMapped) == cudaSuccess &&
              cudaHostGetDevicePointer(reinterpret_cast<void**>(&r.d_done_alias), r.h_done, 0) == cudaSuccess &&

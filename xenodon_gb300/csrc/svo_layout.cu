@@ -127,7 +127,7 @@ int measure_inner_depth(Ctx* c, Volume* v) {
     if (!v->depth_consistent || !v->inner_depth || v->n_inner == 0) return XN_OK;
     uint32_t* d = nullptr;
     uint32_t h = 0xFFFFFFFFu;
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&d), 4, c->stream);
+    cudaError_t e = c->with_room([&] { return cudaMallocAsync(reinterpret_cast<void**>(&d), 4, c->stream); });
     if (e == cudaSuccess) e = cudaMemsetAsync(d, 0, 4, c->stream);
     if (e == cudaSuccess) {
         max_inner_depth_kernel<<<1024, 256, 0, c->stream>>>(v->inner_depth, v->n_inner, d);

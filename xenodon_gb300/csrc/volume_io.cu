@@ -174,7 +174,7 @@ __global__ void check_layout_kernel(const uint32_t* inner, const uint32_t* depth
 int validate_compact_layout(Ctx* c, Volume* v, const char* what) {
     uint32_t* flags = nullptr;
     uint32_t hf[2] = {1, 1};
-    cudaError_t e = cudaMallocAsync(reinterpret_cast<void**>(&flags), 8, c->stream);
+    cudaError_t e = c->with_room([&] { return cudaMallocAsync(reinterpret_cast<void**>(&flags), 8, c->stream); });
     if (e == cudaSuccess) e = cudaMemsetAsync(flags, 0, 8, c->stream);
     if (e == cudaSuccess) {
         check_layout_kernel<<<1024, 256, 0, c->stream>>>(v->inner, v->inner_depth, v->rinner, v->leaves, v->n_inner,

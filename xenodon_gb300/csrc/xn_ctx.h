@@ -59,6 +59,17 @@ struct Ctx {
 
     int sm_count();
 
+    // Device memory that does not come from the pool (arrays, stream-ordered
+    // allocations, graphs): what the pool keeps is given back when it is short.
+    template <class F>
+    cudaError_t with_room(F f) {
+        return pool.with_room([&] {
+            const cudaError_t e = f();
+            if (e == cudaErrorMemoryAllocation) cudaGetLastError();
+            return e;
+        });
+    }
+
     int activate();
     int device_alloc(void** p, uint64_t bytes, const char* what);
     // tracked: every launch that uses the block is on the context's stream or tracked

@@ -41,10 +41,22 @@ public:
 
     explicit BlockPool(const Api& a) : api(a) {}
 
+    // An allocation that does not go through the pool, tried again without the
+    // kept blocks: f returns 0 or the allocator's error.
+    template <class F>
+    auto with_room(F f) {
+        auto e = f();
+        if ((int)e == api.out_of_memory) {
+            trim(0);
+            e = f();
+        }
+        return e;
+    }
+
     // 0, OVER_BUDGET or the allocator's error.
     int alloc(void** p, uint64_t bytes) {
         *p = nullptr;
-        uint64_t size = budget ? bytes : rounded(bytes);
+        const uint64_t size = budget ? bytes : rounded(bytes);
         {
             std::lock_guard<std::mutex> lk(mu);
             if (!admit(bytes)) return OVER_BUDGET;
@@ -63,19 +75,18 @@ public:
             }
             make_room();
         }
-        int e = api.alloc(p, size);
-        if (e == api.out_of_memory) {  // without the kept blocks, and without the rounding
-            trim(0);
-            size = bytes;
-            e = api.alloc(p, size);
-        }
+        uint64_t got = 0;
+        const int e = with_room([&] {  // the second time without the rounding
+            got = got ? bytes : size;
+            return api.alloc(p, got);
+        });
         std::lock_guard<std::mutex> lk(mu);
         if (e) {
             *p = nullptr;
             used -= bytes;
             return e;
         }
-        sizes[*p] = size;
+        sizes[*p] = got;
         return 0;
     }
 
