@@ -34,13 +34,12 @@ int check_config(const xn_batch_config& c) {
     return XN_OK;
 }
 
-// Builds header + jobs into `table`; returns the byte size.
-int fill_table(Ctx* c, const xn_job* jobs, int n, uint32_t tile_w, void* table, uint64_t capacity_bytes,
-               uint64_t* bytes_out, int* spec_out = nullptr) {
-    const uint64_t need = sizeof(BatchHeader) + (uint64_t)n * sizeof(BatchJob);
-    if (need > capacity_bytes) return fail(XN_ERR_ARG, "batch: %d jobs exceed the job table capacity", n);
-    BatchHeader* h = static_cast<BatchHeader*>(table);
-    BatchJob* out = reinterpret_cast<BatchJob*>(h + 1);
+// Builds the header, and the jobs at all[first] .. of an array of `capacity`.
+int fill_table(Ctx* c, const xn_job* jobs, int n, uint32_t tile_w, BatchHeader* h, BatchJob* all, uint64_t capacity,
+               uint32_t first, int* spec_out = nullptr) {
+    if ((uint64_t)first + (uint64_t)n > capacity)
+        return fail(XN_ERR_ARG, "batch: %d jobs exceed the job table capacity", n);
+    BatchJob* out = all + first;
     const uint32_t tile_h = 32 / tile_w;
     unsigned long long tiles = 0;
     for (int i = 0; i < n; ++i) {
@@ -62,9 +61,8 @@ int fill_table(Ctx* c, const xn_job* jobs, int n, uint32_t tile_w, void* table, 
         if (spec_out) *spec_out = i == 0 ? sp : (*spec_out == sp ? sp : XN_BATCH_ANY);
     }
     h->n_jobs = (uint32_t)n;
-    h->pad = 0;
+    h->first = first;
     h->total_tiles = tiles;
-    *bytes_out = need;
     return XN_OK;
 }
 
@@ -181,14 +179,14 @@ int render_batch_locked(Ctx* c, const xn_job* jobs, int n, const xn_batch_config
 }
 
 int render_batch_one(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& cfg, cudaStream_t s) {
-    const uint64_t cap = sizeof(BatchHeader) + (uint64_t)n * sizeof(BatchJob);
-    int r = ensure_batch_staging(c, cap);
+    const uint64_t bytes = sizeof(BatchHeader) + (uint64_t)n * sizeof(BatchJob);
+    int r = ensure_batch_staging(c, bytes);
     if (r) return r;
     cudaError_t e = cudaEventSynchronize(c->batch_copied);  // the previous table left the staging buffer
     if (e != cudaSuccess) return cuda_fail(e, "xn_render_batch: staging");
-    uint64_t bytes = 0;
     int spec = XN_BATCH_ANY;
-    if ((r = fill_table(c, jobs, n, cfg.tile_width, c->batch_host, c->batch_host_bytes, &bytes, &spec))) return r;
+    BatchHeader* h = static_cast<BatchHeader*>(c->batch_host);
+    if ((r = fill_table(c, jobs, n, cfg.tile_width, h, reinterpret_cast<BatchJob*>(h + 1), (uint64_t)n, 0, &spec))) return r;
     // XN_BATCH_GENERIC=1 keeps the generic form (same results)
     if (generic_forced()) spec = XN_BATCH_ANY;
     const uint64_t queue_off = (bytes + 255) & ~255ull;
@@ -199,7 +197,7 @@ int render_batch_one(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& c
     e = cudaMemcpyAsync(d, c->batch_host, bytes, cudaMemcpyHostToDevice, s);
     if (e == cudaSuccess) e = cudaEventRecord(c->batch_copied, s);
     if (e == cudaSuccess) e = cudaMemsetAsync(queue, 0, 8, s);
-    const uint64_t total_tiles = static_cast<const BatchHeader*>(c->batch_host)->total_tiles;
+    const uint64_t total_tiles = h->total_tiles;
     const uint32_t warps = cfg.block_threads / 32;
     const uint64_t grid = cfg.chunk ? resident_blocks(c, cfg) : (total_tiles + warps - 1) / warps;
     if (grid == 0) {
@@ -211,7 +209,8 @@ int render_batch_one(Ctx* c, const xn_job* jobs, int n, const xn_batch_config& c
         return fail(XN_ERR_ARG, "xn_render_batch: too many tiles for one grid; use a queue chunk >= 1");
     }
     if (e == cudaSuccess)
-        e = launch_batch(d, queue, c->d_err, cfg.tile_width, cfg.block_threads, (uint32_t)grid, cfg.chunk, spec, s);
+        e = launch_batch(static_cast<const BatchHeader*>(d),
+                         reinterpret_cast<const BatchJob*>(static_cast<const BatchHeader*>(d) + 1), queue, c->d_err, cfg.tile_width, cfg.block_threads, (uint32_t)grid, cfg.chunk, spec, s);
     const cudaError_t ef = cudaFreeAsync(d, s);
     if (e == cudaSuccess) e = ef;
     return e == cudaSuccess ? XN_OK : cuda_fail(e, "xn_render_batch");
@@ -324,22 +323,30 @@ XN_API int xn_autotune_batch(xn_ctx* h, const xn_job* jobs, int n, void* stream,
 
 // ------------------------------------------------------------------ graphs
 
-// A batch graph captures one launch per kernel form, each over its own
-// segment of the job table (a form without jobs exits at once), or with
-// XN_BATCH_GENERIC=1 one generic launch over the whole table.
+// A batch graph captures one launch per kernel form, each with a header of its
+// own and its jobs one after the other in one array, or with XN_BATCH_GENERIC=1
+// one generic launch over them all.  The launches of forms that a batch does
+// not have are switched off in the instantiated graph (a launch without jobs
+// takes 1.7 us), which costs host time only where a batch has other forms than
+// the one before.  Four 64x64 frames of a 64^3 octree, us a replay: esvo 115
+// with ten launches and ten full tables, 102 with seven, 74 with its own; four
+// traversals 279, 459 (svo-df by the warp there) and 255.
 struct xn_batch_graph {
     Ctx* ctx;
     cudaStream_t stream;
     xn_batch_config cfg;
     bool split = true;
     int capacity;
-    uint64_t seg_bytes;    // one form's segment: header + capacity jobs
-    uint64_t table_bytes;  // all segments
+    uint64_t jobs_at;      // the headers' bytes
+    uint64_t table_bytes;  // headers and jobs
     struct Slot {
         void* host = nullptr;
         void* dev = nullptr;
         unsigned long long* queue = nullptr;
+        cudaGraph_t graph = nullptr;  // of `launch`
         cudaGraphExec_t exec = nullptr;
+        cudaGraphNode_t launch[XN_BATCH_FORMS] = {};
+        uint32_t on = 0;  // bit f: form f's launch is switched on
         cudaEvent_t done = nullptr;
         bool pending = false;
     } slot[2];
@@ -356,6 +363,7 @@ void destroy_graph(xn_batch_graph* g) {
             cudaEventDestroy(s.done);
         }
         if (s.exec) cudaGraphExecDestroy(s.exec);
+        if (s.graph) cudaGraphDestroy(s.graph);
         if (s.host) cudaFreeHost(s.host);
         c->device_free(s.dev, g->table_bytes);
         c->device_free(s.queue, 64 * XN_BATCH_FORMS);
@@ -385,8 +393,8 @@ XN_API int xn_batch_graph_create(xn_ctx* h, int capacity, const xn_batch_config*
     if (g->cfg.chunk == 0) g->cfg.chunk = 1;  // the tile count changes per replay: graphs use the queue form
     g->capacity = capacity;
     g->split = !generic_forced();
-    g->seg_bytes = (sizeof(BatchHeader) + (uint64_t)capacity * sizeof(BatchJob) + 255) & ~255ull;
-    g->table_bytes = g->seg_bytes * (g->split ? XN_BATCH_FORMS : 1);
+    g->jobs_at = (XN_BATCH_FORMS * sizeof(BatchHeader) + 255) & ~255ull;
+    g->table_bytes = g->jobs_at + (uint64_t)capacity * sizeof(BatchJob);
     if ((r = check_config(g->cfg))) {
         delete g;
         return r;
@@ -408,13 +416,25 @@ XN_API int xn_batch_graph_create(xn_ctx* h, int capacity, const xn_batch_config*
         cudaMemcpyAsync(sl.dev, sl.host, g->table_bytes, cudaMemcpyHostToDevice, cap);
         cudaMemsetAsync(sl.queue, 0, 64 * XN_BATCH_FORMS, cap);
         const int n_launch = g->split ? XN_BATCH_FORMS : 1;
-        for (int f = 0; f < n_launch; ++f)
-            launch_batch(static_cast<char*>(sl.dev) + f * g->seg_bytes, sl.queue + f * 8, c->d_err, g->cfg.tile_width,
-                         g->cfg.block_threads, blocks, g->cfg.chunk, g->split ? f : XN_BATCH_ANY, cap);
-        cudaGraph_t graph = nullptr;
-        e = cudaStreamEndCapture(cap, &graph);
-        if (e == cudaSuccess) e = c->with_room([&] { return cudaGraphInstantiate(&sl.exec, graph, 0); });
-        if (graph) cudaGraphDestroy(graph);
+        for (int f = 0; f < n_launch; ++f) {
+            launch_batch(static_cast<const BatchHeader*>(sl.dev) + f,
+                         reinterpret_cast<const BatchJob*>(static_cast<const char*>(sl.dev) + g->jobs_at),
+                         sl.queue + f * 8, c->d_err, g->cfg.tile_width, g->cfg.block_threads, blocks, g->cfg.chunk,
+                         g->split ? f : XN_BATCH_ANY, cap);
+            // the launch's node is the one that what comes next would depend on
+            cudaStreamCaptureStatus st;
+            const cudaGraphNode_t* last = nullptr;
+            size_t n_last = 0;
+            if (cudaStreamGetCaptureInfo(cap, &st, nullptr, nullptr, &last, nullptr, &n_last) == cudaSuccess &&
+                n_last == 1)
+                sl.launch[f] = last[0];
+            else
+                e = cudaErrorUnknown;
+            sl.on |= 1u << f;
+        }
+        const cudaError_t ec = cudaStreamEndCapture(cap, &sl.graph);
+        if (e == cudaSuccess) e = ec;
+        if (e == cudaSuccess) e = c->with_room([&] { return cudaGraphInstantiate(&sl.exec, sl.graph, 0); });
     }
     if (cap) cudaStreamDestroy(cap);
     if (e != cudaSuccess || r) {
@@ -434,23 +454,33 @@ XN_API int xn_batch_graph_launch(xn_batch_graph* g, const xn_job* jobs, int n) {
     if (r) return r;
     auto& sl = g->slot[g->next];
     if (sl.pending) cudaEventSynchronize(sl.done);  // this slot's previous batch has finished
-    uint64_t bytes = 0;
+    BatchHeader* headers = static_cast<BatchHeader*>(sl.host);
+    BatchJob* all = reinterpret_cast<BatchJob*>(static_cast<char*>(sl.host) + g->jobs_at);
+    cudaError_t e = cudaSuccess;
     if (g->split) {
         std::vector<int> forms;
         if ((r = forms_of(c, jobs, n, forms))) return r;
         std::vector<xn_job> part;
+        uint32_t first = 0;
         for (int f = 0; f < XN_BATCH_FORMS; ++f) {
             part.clear();
             for (int i = 0; i < n; ++i)
                 if (forms[i] == f) part.push_back(jobs[i]);
-            if ((r = fill_table(c, part.data(), (int)part.size(), g->cfg.tile_width,
-                                static_cast<char*>(sl.host) + f * g->seg_bytes, g->seg_bytes, &bytes)))
+            if ((r = fill_table(c, part.data(), (int)part.size(), g->cfg.tile_width, headers + f, all,
+                                (uint64_t)g->capacity, first)))
                 return r;
+            first += (uint32_t)part.size();
+            const uint32_t bit = 1u << f, want = part.empty() ? 0u : bit;
+            if ((sl.on & bit) != want) {
+                e = cudaGraphNodeSetEnabled(sl.exec, sl.launch[f], want != 0);
+                if (e != cudaSuccess) return cuda_fail(e, "xn_batch_graph_launch: forms");
+                sl.on ^= bit;
+            }
         }
-    } else if ((r = fill_table(c, jobs, n, g->cfg.tile_width, sl.host, g->table_bytes, &bytes))) {
+    } else if ((r = fill_table(c, jobs, n, g->cfg.tile_width, headers, all, (uint64_t)g->capacity, 0))) {
         return r;
     }
-    cudaError_t e = cudaGraphLaunch(sl.exec, g->stream);
+    e = cudaGraphLaunch(sl.exec, g->stream);
     launched(c, jobs, n, g->stream);
     if (e == cudaSuccess) e = cudaEventRecord(sl.done, g->stream);
     if (e != cudaSuccess) return cuda_fail(e, "xn_batch_graph_launch");

@@ -2085,6 +2085,7 @@ __global__ void __launch_bounds__(1024, batch_min_blocks(SPEC)) batch_kernel(con
     const uint32_t lane = threadIdx.x & 31u;
     const unsigned long long total = hdr->total_tiles;
     const uint32_t n = hdr->n_jobs;
+    jobs += hdr->first;
     uint32_t err = 0;
     for (;;) {
         unsigned long long base = 0;
@@ -2126,6 +2127,7 @@ __global__ void __launch_bounds__(1024, batch_min_blocks(SPEC)) batch_grid_kerne
     const unsigned long long t =
         (unsigned long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (t >= hdr->total_tiles) return;
+    jobs += hdr->first;
     uint32_t lo = 0, hi = hdr->n_jobs;  // last job whose first tile is <= t
     while (hi - lo > 1) {
         const uint32_t mid = (lo + hi) >> 1;
@@ -2145,10 +2147,8 @@ __global__ void __launch_bounds__(1024, batch_min_blocks(SPEC)) batch_grid_kerne
 }
 
 template <int TW, int SPEC>
-static cudaError_t launch_batch_tws(const void* table, unsigned long long* q, uint32_t* err, uint32_t threads,
-                                    uint32_t blocks, uint32_t chunk, cudaStream_t s) {
-    const BatchHeader* hdr = static_cast<const BatchHeader*>(table);
-    const BatchJob* jobs = reinterpret_cast<const BatchJob*>(hdr + 1);
+static cudaError_t launch_batch_tws(const BatchHeader* hdr, const BatchJob* jobs, unsigned long long* q, uint32_t* err,
+                                    uint32_t threads, uint32_t blocks, uint32_t chunk, cudaStream_t s) {
     const size_t smem = (size_t)batch_rows(SPEC) * 4 * threads;
     if (chunk == 0) {
         // queue-less form: one warp per tile; `blocks` is the grid for all tiles
@@ -2170,31 +2170,33 @@ static cudaError_t launch_batch_tws(const void* table, unsigned long long* q, ui
 }
 
 template <int TW>
-static cudaError_t launch_batch_tw(const void* table, unsigned long long* q, uint32_t* err, uint32_t threads,
-                                   uint32_t blocks, uint32_t chunk, int spec, cudaStream_t s) {
+static cudaError_t launch_batch_tw(const BatchHeader* hdr, const BatchJob* jobs, unsigned long long* q, uint32_t* err,
+                                   uint32_t threads, uint32_t blocks, uint32_t chunk, int spec, cudaStream_t s) {
     switch (spec) {
-    case XN_BATCH_DDA_TEX_NORM: return launch_batch_tws<TW, XN_BATCH_DDA_TEX_NORM>(table, q, err, threads, blocks, chunk, s);
-    case XN_BATCH_DDA_TEX_RAW: return launch_batch_tws<TW, XN_BATCH_DDA_TEX_RAW>(table, q, err, threads, blocks, chunk, s);
-    case XN_BATCH_ESVO: return launch_batch_tws<TW, XN_BATCH_ESVO>(table, q, err, threads, blocks, chunk, s);
-    case XN_BATCH_NAIVE: return launch_batch_tws<TW, XN_BATCH_NAIVE>(table, q, err, threads, blocks, chunk, s);
-    case XN_BATCH_DF: return launch_batch_tws<TW, XN_BATCH_DF>(table, q, err, threads, blocks, chunk, s);
-    case XN_BATCH_DF_STEPS: return launch_batch_tws<TW, XN_BATCH_DF_STEPS>(table, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_DDA_TEX_NORM:
+        return launch_batch_tws<TW, XN_BATCH_DDA_TEX_NORM>(hdr, jobs, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_DDA_TEX_RAW:
+        return launch_batch_tws<TW, XN_BATCH_DDA_TEX_RAW>(hdr, jobs, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_ESVO: return launch_batch_tws<TW, XN_BATCH_ESVO>(hdr, jobs, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_NAIVE: return launch_batch_tws<TW, XN_BATCH_NAIVE>(hdr, jobs, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_DF: return launch_batch_tws<TW, XN_BATCH_DF>(hdr, jobs, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_DF_STEPS: return launch_batch_tws<TW, XN_BATCH_DF_STEPS>(hdr, jobs, q, err, threads, blocks, chunk, s);
     case XN_BATCH_ESVO_SHALLOW:
-        return launch_batch_tws<TW, XN_BATCH_ESVO_SHALLOW>(table, q, err, threads, blocks, chunk, s);
+        return launch_batch_tws<TW, XN_BATCH_ESVO_SHALLOW>(hdr, jobs, q, err, threads, blocks, chunk, s);
     case XN_BATCH_NAIVE_SHALLOW:
-        return launch_batch_tws<TW, XN_BATCH_NAIVE_SHALLOW>(table, q, err, threads, blocks, chunk, s);
-    case XN_BATCH_ROPE: return launch_batch_tws<TW, XN_BATCH_ROPE>(table, q, err, threads, blocks, chunk, s);
-    default: return launch_batch_tws<TW, XN_BATCH_ANY>(table, q, err, threads, blocks, chunk, s);
+        return launch_batch_tws<TW, XN_BATCH_NAIVE_SHALLOW>(hdr, jobs, q, err, threads, blocks, chunk, s);
+    case XN_BATCH_ROPE: return launch_batch_tws<TW, XN_BATCH_ROPE>(hdr, jobs, q, err, threads, blocks, chunk, s);
+    default: return launch_batch_tws<TW, XN_BATCH_ANY>(hdr, jobs, q, err, threads, blocks, chunk, s);
     }
 }
 
-cudaError_t launch_batch(const void* table, unsigned long long* q, uint32_t* err, uint32_t tile_w,
+cudaError_t launch_batch(const BatchHeader* hdr, const BatchJob* jobs, unsigned long long* q, uint32_t* err, uint32_t tile_w,
                          uint32_t threads, uint32_t blocks, uint32_t chunk, int spec, cudaStream_t s) {
     switch (tile_w) {
-    case 4: return launch_batch_tw<4>(table, q, err, threads, blocks, chunk, spec, s);
-    case 16: return launch_batch_tw<16>(table, q, err, threads, blocks, chunk, spec, s);
-    case 32: return launch_batch_tw<32>(table, q, err, threads, blocks, chunk, spec, s);
-    default: return launch_batch_tw<8>(table, q, err, threads, blocks, chunk, spec, s);
+    case 4: return launch_batch_tw<4>(hdr, jobs, q, err, threads, blocks, chunk, spec, s);
+    case 16: return launch_batch_tw<16>(hdr, jobs, q, err, threads, blocks, chunk, spec, s);
+    case 32: return launch_batch_tw<32>(hdr, jobs, q, err, threads, blocks, chunk, spec, s);
+    default: return launch_batch_tw<8>(hdr, jobs, q, err, threads, blocks, chunk, spec, s);
     }
 }
 

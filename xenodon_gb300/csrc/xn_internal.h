@@ -109,7 +109,7 @@ struct alignas(16) BatchJob {
 };
 
 struct alignas(16) BatchHeader {
-    uint32_t n_jobs, pad;
+    uint32_t n_jobs, first;  // its jobs are `first` .. of the launch's array
     unsigned long long total_tiles;
 };
 
@@ -123,10 +123,10 @@ enum { XN_BATCH_ANY = 0, XN_BATCH_DDA_TEX_NORM, XN_BATCH_DDA_TEX_RAW, XN_BATCH_E
 // The form a job needs (XN_BATCH_*).
 int batch_spec(const BatchJob& j);
 // Launches the persistent kernel over a job table already in device memory
-// (header followed by the jobs).  tile_w is the warp tile's width in pixels
+// (a header, and the array its jobs are in).  tile_w is the warp tile's width in pixels
 // (4, 8, 16 or 32; height 32/tile_w); spec is the form every job shares, or
 // XN_BATCH_ANY.
-cudaError_t launch_batch(const void* d_table, unsigned long long* d_queue, uint32_t* d_err, uint32_t tile_w,
+cudaError_t launch_batch(const BatchHeader* d_header, const BatchJob* d_jobs, unsigned long long* d_queue, uint32_t* d_err, uint32_t tile_w,
                          uint32_t threads, uint32_t blocks, uint32_t chunk, int spec, cudaStream_t s);
 int batch_kernel_blocks_per_sm(uint32_t tile_w, uint32_t block_threads);
 
