@@ -14,8 +14,6 @@
 
 namespace xn {
 
-int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_params* p, RenderLaunch& L);
-
 namespace {
 
 uint32_t traversal_mask(const xn_job* jobs, int n) {
@@ -135,7 +133,7 @@ int render_plain(Ctx* c, const xn_job* jobs, int n, cudaStream_t s) {
         const Volume* v = reinterpret_cast<const Volume*>(jobs[i].volume);
         if (v->ctx != c) return fail(XN_ERR_ARG, "batch: job %d uses a volume of another context", i);
         RenderLaunch L;
-        int r = make_launch(v, jobs[i].traversal, &jobs[i].camera, &jobs[i].params, L);
+        int r = make_launch(v, jobs[i].traversal, &jobs[i].camera, &jobs[i].params, L, c->streams_in_use(s));
         if (r) return r;
         L.d_rgba = jobs[i].d_rgba;
         L.d_err_word = c->d_err;

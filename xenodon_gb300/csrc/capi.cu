@@ -68,6 +68,24 @@ void Ctx::device_free(void* p, uint64_t bytes, bool tracked) {
     pool.free(p, bytes, tracked && bytes >= BlockPool::SMALLEST && wait_launches());
 }
 
+uint32_t Ctx::streams_in_use(cudaStream_t s) {
+    std::lock_guard<std::mutex> lk(launch_mu);
+    ++frames;
+    Recent* mine = nullptr;
+    uint32_t n = 0;
+    for (Recent& r : recent) {
+        if (r.turn && r.stream == s) mine = &r;
+        else if (r.turn && frames - r.turn < RECENT_FRAMES) ++n;
+    }
+    if (!mine) {
+        mine = &recent[0];
+        for (Recent& r : recent)
+            if (r.turn < mine->turn) mine = &r;
+    }
+    *mine = {s, frames};
+    return n + 1;
+}
+
 // 0.3 us of host time (a launch with it 3.4 us, without 3.1).
 bool Ctx::track_launch(cudaStream_t s) {
     if (s == stream) return true;
@@ -561,6 +579,14 @@ namespace xn {
 // and svo-rope 1.45-1.7x, the others 1.1-1.2x), from farther away 24 (160x120
 // with warps of 8: 1.1-1.3x) and 48 (139x139 with warps of 4: 1.4-2.5x; 256x256
 // of 16: 1.06-1.3x).  At twice these counts some lose 10-40 %.
+//
+// `rays` are the frame's times the streams that the context's last 64 frames
+// went to, as frames on other streams run beside it.  16 streams of 160x120
+// frames of a 256^3 gas field, us a frame with 32 rays a warp throughout, by
+// this rule, and by the frame's own rays alone: esvo from outside 41, 37, 177;
+// svo-rope 44, 44, 124; dda 11, 6, 24; from inside 42, 39, 71; 25, 25, 39; 7.7,
+// 6.1, 9.2.  On 4 streams no frame of 96x96 to 256x256 was slower than with 32
+// rays; esvo from outside 96, 95, 177.
 static uint32_t narrow_warps(uint64_t rays, int sms, bool large, float zoom) {
     const uint32_t limit = zoom < 0.77f ? (large ? 48 : 24) : zoom < 1.15f ? (large ? 27 : 16) : 8;
     for (uint32_t n = 4; n > 0; --n)
@@ -568,7 +594,8 @@ static uint32_t narrow_warps(uint64_t rays, int sms, bool large, float zoom) {
     return 0;
 }
 
-int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_params* p, RenderLaunch& L) {
+int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_params* p, RenderLaunch& L,
+                uint32_t streams) {
     if (traversal < XN_DDA || traversal > XN_SVO_ROPE) return fail(XN_ERR_ARG, "invalid traversal %d", traversal);
     if (traversal == XN_DDA && v->kind != XN_VOLUME_GRID)
         return fail(XN_ERR_ARG, "traversal 'dda' requires a grid volume (tiff)");
@@ -612,7 +639,8 @@ int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_p
             d2 += c * c;
             f2 += L.forward[i] * L.forward[i];
         }
-        L.narrow = narrow_warps((uint64_t)L.out_w * L.out_h, v->ctx->sm_count(), side >= (grid ? 128u : 256u),
+        const char* nw = std::getenv("XN_NARROW_WARPS");  // 0: warps of 32 rays throughout
+        L.narrow = nw && nw[0] == '0' ? 0 : narrow_warps((uint64_t)L.out_w * L.out_h * streams, v->ctx->sm_count(), side >= (grid ? 128u : 256u),
                                 std::sqrt(f2 / d2));
     }
     if (v->kind == XN_VOLUME_GRID) {
@@ -686,7 +714,7 @@ XN_API int xn_render_device(xn_ctx* h, const xn_volume* vh, int traversal, const
     const Volume* v = reinterpret_cast<const Volume*>(vh);
     if (v->ctx != c) return fail(XN_ERR_ARG, "xn_render_device: volume belongs to another context");
     RenderLaunch L;
-    int r = make_launch(v, traversal, cam, params, L);
+    int r = make_launch(v, traversal, cam, params, L, c->streams_in_use(static_cast<cudaStream_t>(stream)));
     if (r) return r;
     L.d_rgba = d_rgba;
     L.d_emission = d_emission;
@@ -706,7 +734,7 @@ XN_API int xn_render(xn_ctx* h, const xn_volume* vh, int traversal, const xn_cam
     const Volume* v = reinterpret_cast<const Volume*>(vh);
     if (v->ctx != c) return fail(XN_ERR_ARG, "xn_render: volume belongs to another context");
     RenderLaunch L;
-    int r = make_launch(v, traversal, cam, params, L);
+    int r = make_launch(v, traversal, cam, params, L, c->streams_in_use(c->stream));
     if (r) return r;
     std::lock_guard<std::mutex> lk(c->mu);
     if ((r = c->activate())) return r;

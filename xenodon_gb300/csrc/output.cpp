@@ -22,8 +22,6 @@
 
 namespace xn {
 
-int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_params* p, RenderLaunch& L);
-
 struct Output {
     Ctx* ctx = nullptr;
     uint64_t max_pixels = 0;
@@ -88,7 +86,7 @@ XN_API int xn_output_render(xn_output* oh, const xn_volume* vh, int traversal, c
     if (o->pending) return fail(XN_ERR_STATE, "xn_output_render: the previous render was not waited for");
     if (flags & ~XN_OUTPUT_DISCARD) return fail(XN_ERR_ARG, "xn_output_render: unknown flags 0x%x", flags);
     RenderLaunch L;
-    int r = make_launch(v, traversal, cam, params, L);
+    int r = make_launch(v, traversal, cam, params, L, c->streams_in_use(c->stream));
     if (r) return r;
     const uint64_t npix = (uint64_t)L.out_w * L.out_h;
     if (npix > o->max_pixels)

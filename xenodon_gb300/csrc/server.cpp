@@ -52,7 +52,6 @@
 #include "xn_internal.h"
 
 namespace xn {
-int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_params* p, RenderLaunch& L);
 }  // namespace xn
 
 using xn::fail;

@@ -54,6 +54,17 @@ struct Ctx {
     std::vector<Launch> launches;
     std::vector<cudaEvent_t> spare_events;
     uint64_t launch_turn = 0;
+
+    // Streams of the last frames, single launches each: how many of them are in
+    // use side by side.
+    struct Recent {
+        cudaStream_t stream;
+        uint64_t turn;  // 0: free
+    };
+    static constexpr uint64_t RECENT_FRAMES = 64;
+    Recent recent[32] = {};
+    uint64_t frames = 0;
+    uint32_t streams_in_use(cudaStream_t s);  // before a frame's launch on s
     bool track_launch(cudaStream_t s);  // false: the end of this launch is not known
     bool wait_launches();               // waits for the context's stream and all tracked launches; false: not known
 
@@ -154,6 +165,12 @@ struct SubBuild {
 int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, uint32_t dz, int type, int heuristic,
                      double threshold, uint32_t** d_nodes, uint64_t* d_nodes_bytes, xn_build_stats* stats,
                      Volume* layout = nullptr, bool lean = false, SubBuild* sub = nullptr);
+
+// A frame as the kernels take it.  streams: in use side by side (a frame of
+// `streams` times the pixels fills as much of the GPU).
+struct RenderLaunch;
+int make_launch(const Volume* v, int traversal, const xn_camera* cam, const xn_params* p, RenderLaunch& L,
+                uint32_t streams = 1);
 
 int fail(int code, const char* fmt, ...) __attribute__((format(printf, 2, 3)));
 int cuda_fail(cudaError_t e, const char* what);
