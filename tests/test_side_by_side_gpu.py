@@ -75,3 +75,29 @@ def test_wide_warps_by_switch(ctx, scene, monkeypatch):
         monkeypatch.setenv("XN_NARROW_WARPS", "0")
         assert np.array_equal(ctx.render(vol, trav, cam, p)[0], want)
         monkeypatch.delenv("XN_NARROW_WARPS")
+
+
+def test_frames_that_were_waited_for_are_not_side_by_side(ctx, scene):
+    """A program that also renders to host memory, which waits for the frame:
+    its frames on a stream take as long as without."""
+    import time
+    import torch
+    vol, cam, p = scene
+    s = torch.cuda.Stream()
+    out = torch.zeros((120, 160, 4), dtype=torch.uint8, device="cuda")
+
+    def frames(with_host):
+        times = []
+        for _ in range(90):
+            if with_host:
+                ctx.render(vol, "svo-naive", cam, p)
+            torch.cuda.synchronize()
+            t = time.perf_counter()
+            ctx.render_device(vol, "svo-naive", cam, p, out.data_ptr(), None, None, s.cuda_stream)
+            torch.cuda.synchronize()
+            times.append(time.perf_counter() - t)
+        return sorted(times)[75]
+
+    frames(False)
+    alone = frames(False)
+    assert frames(True) <= 1.1 * alone

@@ -86,6 +86,12 @@ uint32_t Ctx::streams_in_use(cudaStream_t s) {
     return n + 1;
 }
 
+void Ctx::stream_idle(cudaStream_t s) {
+    std::lock_guard<std::mutex> lk(launch_mu);
+    for (Recent& r : recent)
+        if (r.stream == s) r.turn = 0;
+}
+
 // 0.3 us of host time (a launch with it 3.4 us, without 3.1).
 bool Ctx::track_launch(cudaStream_t s) {
     if (s == stream) return true;
@@ -756,6 +762,7 @@ XN_API int xn_render(xn_ctx* h, const xn_volume* vh, int traversal, const xn_cam
     uint32_t err_bits = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&err_bits, c->d_err, sizeof(uint32_t), cudaMemcpyDeviceToHost, c->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(c->stream);
+    c->stream_idle(c->stream);
     if (e != cudaSuccess) return cuda_fail(e, "xn_render");
     if (kernel_ms) {
         e = cudaEventElapsedTime(kernel_ms, c->ev0, c->ev1);

@@ -65,6 +65,7 @@ struct Ctx {
     Recent recent[32] = {};
     uint64_t frames = 0;
     uint32_t streams_in_use(cudaStream_t s);  // before a frame's launch on s
+    void stream_idle(cudaStream_t s);         // its frames have been waited for
     bool track_launch(cudaStream_t s);  // false: the end of this launch is not known
     bool wait_launches();               // waits for the context's stream and all tracked launches; false: not known
 
