@@ -53,6 +53,11 @@ constexpr uint8_t F_LEAF = 1, F_INSIDE = 2;
 constexpr int BT = 128;          // a scan block: 4 warps, each two octants (8^3 voxels) of the brick that are neighbours in x
 constexpr uint32_t ROOT_BIT = 256;
 constexpr uint64_t TOP_CELLS = 1024;
+// Levels whose cells' std-dev decisions may take the reference's loop over the
+// cell's voxels, a thread each, are spread over the GPU from here, in blocks of
+// as many: with all 512 cells of 32^3 voxels of a 256^3 grid at the threshold
+// the build takes 19 ms; in one block their loops alone took 76.
+constexpr uint64_t TOP_LOOPS = 64;
 
 // Octants o, groups g (4^3 voxels, eight an octant) and cells m (2^3 voxels,
 // 64 an octant, m = 8 g + child) are in child order: x is the high digit.
@@ -206,7 +211,7 @@ __device__ __forceinline__ bool cell_internal(const Levels& a, uint32_t x, uint3
     const unsigned long long E = (unsigned long long)n * p.q -
                                  ((unsigned long long)s0 * s0 + (unsigned long long)s1 * s1 +
                                   (unsigned long long)s2 * s2 + (unsigned long long)s3 * s3);
-    bool seq = a.sequential != 0, split;
+    bool split, seq;  // seq: never needed, e <= EXACT_CELL
     if (E == 0) {
         split = 0.0 > a.stddev;  // every voxel equals the mean: the double sum is exactly 0
     } else {
@@ -216,9 +221,8 @@ __device__ __forceinline__ bool cell_internal(const Levels& a, uint32_t x, uint3
         if (ef > lim * 1.001f && lim < 1e30f) split = true;
         else if (ef < lim * 0.999f && lim < 1e30f) split = false;
         else split = stddev_split((double)E, n, a.stddev, seq);
-        seq |= a.sequential != 0;
     }
-    if (seq) {
+    if (a.sequential) {
         const unsigned long long s[4] = {s0, s1, s2, s3};
         split = sequential_split(a.g, x, y, z, e, s, a.stddev);
     }
@@ -600,7 +604,8 @@ __device__ void up_cell(const Levels& a, int d, uint64_t i) {
         out.s2[0] = q;
         bool seq = false;
         split = E == 0 ? 0.0 > a.stddev : stddev_split((double)E, n, a.stddev, seq);
-        if (seq || a.sequential) split = sequential_split(a.g, ox, oy, oz, e, s, a.stddev);
+        // (a cell partly outside is split whatever its deviation)
+        if ((seq && fully) || a.sequential) split = sequential_split(a.g, ox, oy, oz, e, s, a.stddev);
     }
     const bool leaf = !split && fully;
     a.color[cell] = avg;
@@ -652,10 +657,11 @@ __global__ void __launch_bounds__(256) start_kernel(const __grid_constant__ Leve
     report_depth(a, i < a.geo[d].n ? start_cell(a, d, i) : 0u);
 }
 
-// Depths dtop .. 0 up and their children's starts down, in one block.
+// Depths dup .. 0 up, and of depths 0 .. dtop the children's starts down, in one
+// block.
 template <int HEUR>
-__global__ void __launch_bounds__(1024) top_kernel(const __grid_constant__ Levels a, int dtop) {
-    for (int d = dtop; d >= 0; --d) {
+__global__ void __launch_bounds__(1024) top_kernel(const __grid_constant__ Levels a, int dup, int dtop) {
+    for (int d = dup; d >= 0; --d) {
         for (uint64_t i = threadIdx.x; i < a.geo[d].n; i += blockDim.x) up_cell<HEUR>(a, d, i);
         __syncthreads();
     }
@@ -1181,13 +1187,15 @@ cudaError_t brick_scan(const BrickBuild& b, cudaStream_t s) {
     else if (cd) brick_scan_kernel<XN_HEUR_CHANNEL_DIFF, false><<<nb, BT, 0, s>>>(a);
     else if (vec) brick_scan_kernel<XN_HEUR_STD_DEV, true><<<nb, BT, 0, s>>>(a);
     else brick_scan_kernel<XN_HEUR_STD_DEV, false><<<nb, BT, 0, s>>>(a);
-    int d = b.Lb - 1;
-    for (; d >= 0 && b.geo[d].n > TOP_CELLS; --d) {
-        if (cd) up_kernel<XN_HEUR_CHANNEL_DIFF><<<blocks_for(b.geo[d].n, 256), 256, 0, s>>>(a, d);
-        else up_kernel<XN_HEUR_STD_DEV><<<blocks_for(b.geo[d].n, 256), 256, 0, s>>>(a, d);
+    int up = b.Lb - 1;
+    for (; up >= 0 && b.geo[up].n > (cd ? TOP_CELLS : TOP_LOOPS); --up) {
+        if (cd) up_kernel<XN_HEUR_CHANNEL_DIFF><<<blocks_for(b.geo[up].n, 256), 256, 0, s>>>(a, up);
+        else up_kernel<XN_HEUR_STD_DEV><<<blocks_for(b.geo[up].n, TOP_LOOPS), TOP_LOOPS, 0, s>>>(a, up);
     }
-    if (cd) top_kernel<XN_HEUR_CHANNEL_DIFF><<<1, 1024, 0, s>>>(a, d);
-    else top_kernel<XN_HEUR_STD_DEV><<<1, 1024, 0, s>>>(a, d);
+    int d = up;
+    while (d + 1 < b.Lb && b.geo[d + 1].n <= TOP_CELLS) ++d;
+    if (cd) top_kernel<XN_HEUR_CHANNEL_DIFF><<<1, 1024, 0, s>>>(a, up, d);
+    else top_kernel<XN_HEUR_STD_DEV><<<1, 1024, 0, s>>>(a, up, d);
     for (++d; d < b.Lb; ++d) start_kernel<<<blocks_for(b.geo[d].n, 256), 256, 0, s>>>(a, d);
     return cudaGetLastError();
 }

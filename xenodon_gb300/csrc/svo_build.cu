@@ -175,7 +175,8 @@ __global__ void up_level_kernel(UpArgs a) {
         }
         bool seq = false;
         split = E == 0 ? 0.0 > a.stddev : stddev_split((double)E, n, a.stddev, seq);
-        if (seq || a.sequential) split = sequential_split(a.g, ox, oy, oz, e, s, a.stddev);
+        // (a cell partly outside is split whatever its deviation)
+        if ((seq && fully && e > EXACT_CELL) || a.sequential) split = sequential_split(a.g, ox, oy, oz, e, s, a.stddev);
     }
     a.color[i] = avg;
     const bool leaf = (!split && fully) || e == 1;
@@ -575,6 +576,10 @@ struct Scratch {
 
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
 
+// Cells whose decision may take the reference's loop over their voxels, a thread
+// each, are spread over more blocks.
+inline unsigned stddev_block(const LevelGeom& g) { return g.e > EXACT_CELL ? 64 : 256; }
+
 // Exclusive prefix sum of n small counts into u32 (recursive over block sums).
 template <class In>
 int exclusive_scan(Scratch& sc, const In* in, uint64_t n, unsigned* out, cudaStream_t s) {
@@ -785,7 +790,7 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
         a.stddev = threshold;
         a.sequential = heuristic == XN_HEUR_STD_DEV && getenv("XN_BUILD_STDDEV_SEQUENTIAL") != nullptr;
         if (heuristic == XN_HEUR_STD_DEV)
-            up_level_kernel<XN_HEUR_STD_DEV><<<blocks_for(geo[d].n, T), T, 0, s>>>(a);
+            up_level_kernel<XN_HEUR_STD_DEV><<<blocks_for(geo[d].n, stddev_block(geo[d])), stddev_block(geo[d]), 0, s>>>(a);
         else up_level_kernel<XN_HEUR_CHANNEL_DIFF><<<blocks_for(geo[d].n, T), T, 0, s>>>(a);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
     }
@@ -1680,7 +1685,7 @@ int build_static(const uint32_t* d_vox, uint32_t dx, uint32_t dy, uint32_t dz, i
         u.chan_diff = (uint32_t)(uint8_t)threshold;
         u.stddev = threshold;
         if (heuristic == XN_HEUR_STD_DEV)
-            up_level_kernel<XN_HEUR_STD_DEV><<<blocks_for(geo[d].n, T), T, 0, s>>>(u);
+            up_level_kernel<XN_HEUR_STD_DEV><<<blocks_for(geo[d].n, stddev_block(geo[d])), stddev_block(geo[d]), 0, s>>>(u);
         else up_level_kernel<XN_HEUR_CHANNEL_DIFF><<<blocks_for(geo[d].n, T), T, 0, s>>>(u);
         e = cudaGetLastError();
     }

@@ -37,10 +37,18 @@ static __device__ __noinline__ bool sequential_split(const GridDev& g, uint64_t 
     return sqrt(s / nd) > threshold;
 }
 
+// Cells of 2^k voxels a side up to this that lie inside the grid: there the
+// reference's sum is exact in any order.  The mean is a multiple of 2^-3k, so
+// the squares and their sums are multiples of 2^-6k, and with n = 2^3k voxels of
+// four bytes the sum is below n 2^16: 9k + 16 bits, 52 for k = 4.  It is E / n,
+// and the square root below is the reference's own.
+constexpr uint64_t EXACT_CELL = 16;
+
 // Whether the standard deviation sqrt(E)/n, E = n sum(x^2) - sum(x)^2 exact,
 // is above the threshold, as the reference's sequential double sum decides:
 // that sum differs from the exact value by at most (n + 16) 2^-52 relative,
-// and inside that band its own loop decides (seq).
+// and inside that band its own loop decides (seq), but for cells of EXACT_CELL
+// and below.
 static __device__ __forceinline__ bool stddev_split(double E, uint64_t n, double threshold, bool& seq) {
     const double nd = (double)n;
     const double sd = sqrt(E / (nd * nd));
