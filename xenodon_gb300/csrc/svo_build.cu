@@ -572,6 +572,15 @@ struct Scratch {
         *p = static_cast<T*>(v);
         return XN_OK;
     }
+    void free(void* p) {  // before the end of the build
+        for (auto& b : bufs)
+            if (b.first == p) {
+                c->device_free(b.first, b.second);
+                b = bufs.back();
+                bufs.pop_back();
+                return;
+            }
+    }
 };
 
 inline unsigned blocks_for(uint64_t n, unsigned t) { return (unsigned)((n + t - 1) / t); }
@@ -876,8 +885,8 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
 
     if (dag) {
         // ---- DAG: classes depth by depth, deepest first
-        // every depth's classes, the hash table of the largest depth, and the
-        // ranks, in one allocation
+        // every depth's classes; the hash table of the largest depth, given back
+        // before the ranks and the nodes, which are about as large
         std::vector<unsigned long long*> canon(L + 1);
         auto table_size = [&](int d) -> uint64_t {
             const uint64_t count = d < L ? hexist[2 * d] : 8 * hexist[2 * (L - 1) + 1];
@@ -889,7 +898,7 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
         uint8_t* is_rep = nullptr;
         unsigned* ins = nullptr;
         auto plan_dag = [&](unsigned char* base) -> uint64_t {
-            uint64_t used = 0, slots = 1;
+            uint64_t used = 0;
             auto take = [&](uint64_t bytes) -> void* {
                 void* p = base ? base + used : nullptr;
                 used += (bytes + 255) & ~255ull;
@@ -897,20 +906,15 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
             };
             for (int d = 0; d <= L; ++d) {
                 canon[d] = static_cast<unsigned long long*>(take((d < L ? geo[d].n : 8 * geo[L - 1].n) * 8));
-                slots = std::max(slots, table_size(d));
             }
-            // the ranks take the table's place once the classes are known
-            const uint64_t table_at = used;
-            table = static_cast<Slot*>(take(slots * sizeof(Slot)));
-            const uint64_t end = used;
-            used = table_at;
-            is_rep = static_cast<uint8_t*>(take(n_total));
-            ins = static_cast<unsigned*>(take(n_total * 4));
-            return std::max(used, end);
+            return used;
         };
         unsigned char* dag_base = nullptr;
         if ((r = sc.alloc(&dag_base, plan_dag(nullptr), "xn_build_svo: DAG classes"))) return r;
         plan_dag(dag_base);
+        uint64_t slots = 1;
+        for (int d = 0; d <= L; ++d) slots = std::max(slots, table_size(d));
+        if ((r = sc.alloc(&table, slots, "xn_build_svo: DAG table"))) return r;
         auto level_of = [&](int d) {
             DagLevel a{};
             a.depth = d;
@@ -943,6 +947,10 @@ int build_svo_device(Ctx* c, const uint32_t* d_vox, uint32_t dx, uint32_t dy, ui
             }
         }
         if (e != cudaSuccess) return cuda_fail(e, "xn_build_svo: DAG classes");
+        sc.free(table);
+        if ((r = sc.alloc(&is_rep, n_total, "xn_build_svo: DAG ranks")) ||
+            (r = sc.alloc(&ins, n_total, "xn_build_svo: DAG ranks")))
+            return r;
         e = cudaMemsetAsync(is_rep, 0, n_total, s);
         for (int d = L; d >= 0 && e == cudaSuccess; --d) {
             const uint64_t ids = d < L ? geo[d].n : 8 * geo[L - 1].n;
