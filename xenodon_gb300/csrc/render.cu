@@ -1909,13 +1909,13 @@ __device__ __forceinline__ V3 trace_svo_job(const Acc& a, const Frame& f, V3 rd,
         return trace_naive<false>(a, f.translation, rd, loads, err);
     } else if (TRAV == XN_TRAV_SVO_DF) {
         return trace_df<false>(a, f.translation, rd, loads, err);
-    } else if (TRAV == XN_TRAV_SVO_DF_MASKED) {
-        return trace_df_masked<false, Acc, SharedStacks>(a, f.translation, rd, loads, err, stk);
     }
     return trace_rope<false>(a, f.translation, rd, loads, err);
 }
 
-// One pixel of one job: the same arithmetic as the single-frame kernels.
+// One pixel of a job without a form of its own (XN_BATCH_ANY, batch_spec):
+// linear and bricked grids, reference-layout octrees and the literal svo-df.
+// The same arithmetic as the single-frame kernels.
 __device__ __noinline__ uint32_t render_job_pixel(const BatchJob& J, uint32_t ix, uint32_t iy, uint32_t& err,
                                                   SharedStacks* stk) {
     const Frame f = frame_of(J);
@@ -1928,13 +1928,7 @@ __device__ __noinline__ uint32_t render_job_pixel(const BatchJob& J, uint32_t ix
         const V3 ro = f.translation * side;
         const float ec = __fdiv_rn(voxel_emission_coeff(f, rd), side);
         V3 total;
-        if (J.layout == 1) {
-            total = J.tex_normalized == TEX_NORM
-                        ? trace_dda_tex<false, TEX_NORM>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err)
-                    : J.tex_normalized == TEX_PACKED
-                        ? trace_dda_tex<false, TEX_PACKED>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err)
-                        : trace_dda_tex<false, TEX_RAW>(J.tex, J.dim[0], J.dim[1], J.dim[2], ro, rd, loads, err);
-        } else if (J.layout == 2) {
+        if (J.layout == 2) {
             const BrickGrid g{static_cast<const uint4*>(J.grid), J.dim[0], J.dim[1], J.dim[2], bricks_along(J.dim[0]),
                               bricks_along(J.dim[1])};
             total = trace_dda_brick<false>(g, ro, rd, loads, err);
@@ -1954,19 +1948,8 @@ __device__ __noinline__ uint32_t render_job_pixel(const BatchJob& J, uint32_t ix
             case XN_TRAV_SVO_DF: total = trace_svo_job<XN_TRAV_SVO_DF>(a, f, rd, loads, err, stk); break;
             default: total = trace_svo_job<XN_TRAV_SVO_ROPE>(a, f, rd, loads, err, stk); break;
             }
-        } else if (J.traversal == XN_TRAV_SVO_ROPE) {
-            total = trace_svo_job<XN_TRAV_SVO_ROPE>(RopeNodes{J.rinner, J.inner_depth, J.leaves}, f, rd, loads, err,
-                                                    stk);
         } else {
-            CompactNodes a{J.inner, J.inner_depth};
-            switch (J.traversal) {
-            case XN_TRAV_SVO_NAIVE: total = trace_svo_job<XN_TRAV_SVO_NAIVE>(a, f, rd, loads, err, stk); break;
-            case XN_TRAV_ESVO: total = trace_svo_job<XN_TRAV_ESVO>(a, f, rd, loads, err, stk); break;
-            default:
-                total = J.depth_consistent ? trace_svo_job<XN_TRAV_SVO_DF_MASKED>(a, f, rd, loads, err, stk)
-                                           : trace_svo_job<XN_TRAV_SVO_DF>(a, f, rd, loads, err, stk);
-                break;
-            }
+            total = trace_svo_job<XN_TRAV_SVO_DF>(CompactNodes{J.inner, J.inner_depth}, f, rd, loads, err, stk);
         }
         color = total * voxel_emission_coeff(f, rd);
     }
@@ -1974,7 +1957,7 @@ __device__ __noinline__ uint32_t render_job_pixel(const BatchJob& J, uint32_t ix
 }
 
 // One pixel of a job whose traversal and layout the whole batch shares
-// (BatchSpec): that traversal inlined, the arithmetic of render_job_pixel.
+// (batch_spec): that traversal inlined, the arithmetic of the single frames.
 // Called by every lane of a warp tile (active: the pixel is in the job's
 // output); the svo-df form walks the tree with the whole warp.
 template <int SPEC>
@@ -1996,8 +1979,7 @@ __device__ __forceinline__ uint32_t render_job_pixel_spec(const BatchJob& J, uin
     if (!active) return 0u;
     if constexpr (SPEC == XN_BATCH_ANY) {
         // a mixed batch: the job's own inlined form, chosen per tile (every
-        // lane of a warp tile has the same job); linear grids, reference
-        // layouts and the literal svo-df go through the generic function
+        // lane of a warp tile has the same job)
         switch (J.form) {
         case XN_BATCH_DDA_TEX_NORM: return render_job_pixel_spec<XN_BATCH_DDA_TEX_NORM>(J, ix, iy, true, err, stk);
         case XN_BATCH_DDA_TEX_RAW: return render_job_pixel_spec<XN_BATCH_DDA_TEX_RAW>(J, ix, iy, true, err, stk);
@@ -2046,9 +2028,7 @@ __device__ __forceinline__ uint32_t render_job_pixel_spec(const BatchJob& J, uin
                                                     stk) *
                     voxel_emission_coeff(f, rd);
         } else {
-            constexpr int TRAV = SPEC == XN_BATCH_ESVO ? XN_TRAV_ESVO
-                                 : SPEC == XN_BATCH_NAIVE ? XN_TRAV_SVO_NAIVE
-                                                          : XN_TRAV_SVO_DF_MASKED;
+            constexpr int TRAV = SPEC == XN_BATCH_ESVO ? XN_TRAV_ESVO : XN_TRAV_SVO_NAIVE;
             color = trace_svo_job<TRAV>(CompactNodes{J.inner, J.inner_depth}, f, rd, loads, err, stk) *
                     voxel_emission_coeff(f, rd);
         }
