@@ -156,7 +156,6 @@ __device__ __forceinline__ void part_add(Part& p, uint32_t v, bool valid) {
     }
 }
 
-template <int HEUR>
 __device__ __forceinline__ Part part_empty() {
     return Part{0, 0, 0x00FF00FFu, 0x00FF00FFu, 0, 0, 0};
 }
@@ -336,11 +335,11 @@ __device__ __forceinline__ void scan_octant(const Levels& a, const uint4 q[4], c
         }
     }
     const uint32_t x = OX + pl.cx * 2, y = OY + pl.cy * 2, z = OZ + pl.cz * 2;
-    Part group = part_empty<HEUR>();
+    Part group = part_empty();
     uint32_t in[2];
 #pragma unroll
     for (uint32_t c = 0; c < 2; ++c) {
-        Part p = part_empty<HEUR>();
+        Part p = part_empty();
 #pragma unroll
         for (uint32_t k = 0; k < 8; ++k) {
             const bool valid = WHOLE || (x + 2 * c + (k >> 2) < a.g.dx && y + ((k >> 1) & 1u) < a.g.dy &&

@@ -3,7 +3,10 @@
 //
 // The reference builds top-down and re-scans every voxel once per ancestor
 // level; it inserts nodes in post-order (children 0..7, then the parent),
-// reverses the array and rewrites child indices as `end - index`.  Here:
+// reverses the array and rewrites child indices as `end - index`.  Sparse and
+// rope trees of grids of 16 voxels and more on the longest side are built over
+// bricks (svo_bricks.cu).  Here, for DAGs, whose classes need every depth's
+// cells, and for smaller grids:
 //
 //  1. Bottom-up, one kernel per depth d = L-1 .. 0 over the cells of that depth
 //     (cell extent e = side >> d):
@@ -1604,7 +1607,8 @@ void plan_levels(Arena& a, StaticLevels& p, const LevelGeom* geo, int L, int heu
     p.counters = a.take<unsigned int>(4);
     p.leaf_count = a.take<unsigned long long>(1);
     p.existing = a.take<unsigned long long>(2 * (uint64_t)L);
-    // part of what std-dev builds are admitted by
+    // Eight more bytes for each cell of the largest depth, which nothing uses:
+    // what is admitted does not depend on how the decisions are taken.
     if (heuristic == XN_HEUR_STD_DEV) a.take<unsigned long long>(big);
 }
 

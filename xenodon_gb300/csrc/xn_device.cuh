@@ -131,7 +131,7 @@ struct Frame {
     uint32_t out_w, out_h;
     int32_t disp_x, disp_y;
     uint32_t disp_w, disp_h;
-    uint32_t narrow;  // 0: warps of 32 rays (8x4 pixels); 1: of 16 (4x4); 2: of 8 (4x2)
+    uint32_t narrow;  // warps of 32 >> narrow rays: 8x4 pixels, 4x4, 4x2, 2x2 or 2x1
 };
 
 // resources/common.glsl:45-56 with uv from resources/dda.comp:62-63
