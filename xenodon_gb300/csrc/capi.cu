@@ -63,9 +63,9 @@ int Ctx::device_alloc(void** p, uint64_t bytes, const char* what) {
     return e ? cuda_fail((cudaError_t)e, what) : XN_OK;
 }
 
-void Ctx::device_free(void* p, uint64_t bytes, bool tracked) {
+void Ctx::device_free(void* p, uint64_t bytes, Idle idle) {
     if (!p) return;
-    pool.free(p, bytes, tracked && bytes >= BlockPool::SMALLEST && wait_launches());
+    pool.free(p, bytes, idle == IDLE || (idle == WAIT && bytes >= BlockPool::SMALLEST && wait_launches()));
 }
 
 uint32_t Ctx::streams_in_use(cudaStream_t s) {
@@ -130,6 +130,7 @@ bool Ctx::wait_launches() {
     std::vector<Launch> wait;
     {
         std::lock_guard<std::mutex> lk(launch_mu);
+        if (launches.empty() && e == cudaSuccess) return true;
         wait = launches;
     }
     for (size_t i = 0; i < wait.size() && e == cudaSuccess; ++i) e = cudaEventSynchronize(wait[i].done);
@@ -544,9 +545,9 @@ XN_API int xn_volume_release(xn_volume* h) {
     Ctx* c = v->ctx;
     std::lock_guard<std::mutex> lk(c->mu);
     c->activate();
-    cudaStreamSynchronize(c->stream);
-    c->device_free(v->data, v->bytes, !v->untracked);
-    v->release_layout();
+    const Ctx::Idle idle = v->wait();
+    c->device_free(v->data, v->bytes, idle);
+    v->release_layout(idle);
     if (v->tex) cudaDestroyTextureObject(v->tex);
     if (v->array) {
         cudaFreeArray(v->array);

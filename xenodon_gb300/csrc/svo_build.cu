@@ -562,9 +562,11 @@ struct Scratch {
     Ctx* c;
     std::vector<std::pair<void*, uint64_t>> bufs;
     explicit Scratch(Ctx* c) : c(c) {}
+    // (used on the context's stream alone)
+    Ctx::Idle wait() { return cudaStreamSynchronize(c->stream) == cudaSuccess ? Ctx::IDLE : Ctx::UNKNOWN; }
     ~Scratch() {
-        cudaStreamSynchronize(c->stream);
-        for (auto& b : bufs) c->device_free(b.first, b.second);
+        const Ctx::Idle idle = wait();
+        for (auto& b : bufs) c->device_free(b.first, b.second, idle);
     }
     template <class T>
     int alloc(T** p, uint64_t count, const char* what) {
@@ -578,7 +580,7 @@ struct Scratch {
     void free(void* p) {  // before the end of the build
         for (auto& b : bufs)
             if (b.first == p) {
-                c->device_free(b.first, b.second);
+                c->device_free(b.first, b.second, wait());
                 b = bufs.back();
                 bufs.pop_back();
                 return;

@@ -84,8 +84,10 @@ struct Ctx {
 
     int activate();
     int device_alloc(void** p, uint64_t bytes, const char* what);
-    // tracked: every launch that uses the block is on the context's stream or tracked
-    void device_free(void* p, uint64_t bytes, bool tracked = true);
+    // WAIT: for every launch of the context that may use the block; IDLE: the
+    // caller has; UNKNOWN: not all of them are known.
+    enum Idle { WAIT, IDLE, UNKNOWN };
+    void device_free(void* p, uint64_t bytes, Idle idle = WAIT);
     int ensure_buffer(DeviceBuffer& b, uint64_t bytes, const char* what);
     void release_extra();
 };
@@ -128,12 +130,17 @@ struct Volume {
         if (!ctx->track_launch(s)) untracked = true;
     }
 
+    // Waits for the launches that read the volume, as far as they are known.
+    Ctx::Idle wait() const { return !untracked && ctx->wait_launches() ? Ctx::IDLE : Ctx::UNKNOWN; }
+
     void release_layout() {
-        if (!ctx) return;
-        ctx->device_free(inner, n_inner * 32, !untracked);
-        ctx->device_free(rinner, n_inner * 32, !untracked);
-        ctx->device_free(inner_depth, n_inner * 4, !untracked);
-        ctx->device_free(leaves, n_leaves * 32, !untracked);
+        if (ctx && (inner || rinner || inner_depth || leaves)) release_layout(wait());
+    }
+    void release_layout(Ctx::Idle idle) {
+        ctx->device_free(inner, n_inner * 32, idle);
+        ctx->device_free(rinner, n_inner * 32, idle);
+        ctx->device_free(inner_depth, n_inner * 4, idle);
+        ctx->device_free(leaves, n_leaves * 32, idle);
         inner = rinner = inner_depth = leaves = nullptr;
     }
 };
