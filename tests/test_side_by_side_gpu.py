@@ -99,5 +99,5 @@ def test_frames_that_were_waited_for_are_not_side_by_side(ctx, scene):
         return sorted(times)[75]
 
     frames(False)
-    alone = frames(False)
-    assert frames(True) <= 1.1 * alone
+    alone, host = zip(*((frames(False), frames(True)) for _ in range(3)))
+    assert min(host) <= 1.1 * min(alone)
