@@ -131,7 +131,7 @@ struct Volume {
     }
 
     // Waits for the launches that read the volume, as far as they are known.
-    Ctx::Idle wait() const { return !untracked && ctx->wait_launches() ? Ctx::IDLE : Ctx::UNKNOWN; }
+    Ctx::Idle wait() const { return ctx->wait_launches() && !untracked ? Ctx::IDLE : Ctx::UNKNOWN; }
 
     void release_layout() {
         if (ctx && (inner || rinner || inner_depth || leaves)) release_layout(wait());
